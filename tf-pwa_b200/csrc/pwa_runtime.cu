@@ -464,6 +464,9 @@ int pwa_plan_create(const char* src, size_t src_len, int n_mass, int n_angle, in
   CU(cudaHostGetDevicePointer((void**)&h->d_map, h->h_map, 0));
   CU(cudaHostAlloc(&h->h_map_sc, sizeof(double) * (2 * h->nacc + 2), cudaHostAllocMapped));
   CU(cudaHostGetDevicePointer((void**)&h->d_map_sc, h->h_map_sc, 0));
+  // no call number yet: pinned memory may come back from a closed plan with
+  // that plan's last number in it
+  h->h_map[2 * ncol + 2] = -1.0;
   h->h_map_sc[2 * h->nacc + 1] = -1.0;
   return PWA_OK;
 }
