@@ -26,6 +26,7 @@ mathematics is the reference's chain contraction
 """
 import itertools
 
+from .colcode import ColumnCode
 from .decay_config import polarization_names
 from .kincode import KinCode
 from .plan import split_swap
@@ -830,52 +831,6 @@ class ModelCode:
                     e(f"    {dg}.re += {ig};")
                 e("  }")
 
-    # ------------------------------------------------------------ columns
-    def _emit_columns(self, e):
-        for j in range(self.ncol * self.nout):
-            e(f"  F[{j}] = cmk<R>(R(0), R(0));")
-        for ps in range(self.npass):
-            self._pass = ps
-            self._emit_columns_pass(e)
-        self._pass = 0
-
-    def _emit_columns_pass(self, e):
-        fac = self._factor()
-        for ci, c in enumerate(self.group):
-            e(f"  {{ // chain {ci}: {c}" + (f" (swap {self._pass})" if self._pass else ""))
-            self._emit_chain_common(e, ci)
-            for k in self.chain_columns[ci]:
-                e("  {")
-                pre = {}
-                for facs, po, coefs in self.chain_assign[ci]:
-                    if k not in coefs:
-                        continue
-                    ds = [self._d_name(ci, vi, ia, idl) for (vi, ia, idl, _, _) in facs]
-                    prod = ds[0]
-                    for dn in ds[1:]:
-                        prod = f"cmul({prod}, {dn})"
-                    nm = pre.get(po)
-                    if nm is None:
-                        nm = self._pre_name(ci, po, "Fp")
-                        pre[po] = nm
-                        e(f"  cpx<R> {nm} = cmk<R>(R(0), R(0));")
-                    e(f"  cfma({nm}, {self._coef(coefs[k])}, {prod});")
-                cur = self._emit_align_forward(e, ci, pre, "Fa")
-                if getattr(self, "_noshape", False):
-                    # the column without its chain's lineshapes (they are
-                    # applied per evaluation from the masses)
-                    e(f"  const cpx<R> S = cmk<R>({self._scale_k(ci, k)}, R(0));")
-                else:
-                    e(f"  const cpx<R> S = cscale(BW_c{ci}, {self._scale_k(ci, k)});")
-                for o, nm in cur.items():
-                    j = k * self.nout + self._out(o)
-                    if self._pass == 0:
-                        e(f"  F[{j}] = cmul(S, {nm});")
-                    else:
-                        e(f"  F[{j}] = cadd(F[{j}], cscale(cmul(S, {nm}), {_lit(fac)}));")
-                e("  }")
-            e("  }")
-
     # ------------------------------------------------------------ |A|^2
     def _pdf_source(self):
         """``model_f``: sum |A|^2 (``tf_pwa/amp/core.py:1919-1931``) or, for a
@@ -970,26 +925,11 @@ class ModelCode:
                  "    double* __restrict__ accs) {")
         L += body
         L.append("}\n")
-        body = []
+        # the columns with and without their chains' lineshapes, and the
+        # lineshapes with their log-derivatives from the masses alone
+        # (floating-shape column cache)
         self._mode = "plain"
-        self._emit_loads(body.append)
-        self._emit_columns(body.append)
-        L.append(f"template <typename R, bool LDG = true>\n__device__ __forceinline__ void model_columns(\n{sig},\n"
-                 "    cpx<R>* __restrict__ F) {")
-        L += body
-        L.append("}\n")
-        # columns without lineshapes, and the lineshapes with their
-        # log-derivatives from the masses alone (floating-shape column cache)
-        body = []
-        self._mode = "plain"
-        self._noshape = True
-        self._emit_loads(body.append)
-        self._emit_columns(body.append)
-        self._noshape = False
-        L.append(f"template <typename R, bool LDG = true>\n__device__ __forceinline__ void model_columns_ns(\n{sig},\n"
-                 "    cpx<R>* __restrict__ F) {")
-        L += body
-        L.append("}\n")
+        L.append(ColumnCode(self).source())
         body = []
         self._emit_mass_loads(body.append)
         for ci in range(len(self.group)):

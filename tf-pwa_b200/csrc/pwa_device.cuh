@@ -108,6 +108,15 @@ __device__ __forceinline__ void psincos(double x, double* s, double* c) { sincos
 __device__ __forceinline__ void psincos(float x, float* s, float* c) { sincosf(x, s, c); }
 __device__ __forceinline__ double psqrt(double x) { return sqrt(x); }
 __device__ __forceinline__ float psqrt(float x) { return sqrtf(x); }
+// 1 / sqrt(x): CUDA's rsqrt (1 ulp) is one estimate and its refinement, a
+// division of 1 by sqrt(x) is both of a division and a square root
+__device__ __forceinline__ double prsqrt(double x) {
+#ifdef __CUDACC__
+  return rsqrt(x);
+#else
+  return 1.0 / sqrt(x);
+#endif
+}
 
 // e^{i n x/2} for n = -N..N from one sincos of x/2: out[n+N].
 template <typename R, int N>

@@ -18,8 +18,11 @@
 // pwa_reduce  sums the block partials in a fixed order (one warp per
 //             accumulator), so results are bitwise reproducible.
 // pwa_pdf_*   per-event sum |A|^2 (the forward amplitude, AbsPDF.__call__).
-// pwa_columns_f64  per-event partial-wave columns F_k for the Gram cache.
-// pwa_gram_f64     block partials of M_kl = sum_i w_i sum_o conj(F_ik,o) F_il,o.
+// pwa_gram_fused   block partials of M_kl = sum_i w_i sum_o conj(F_ik,o) F_il,o,
+//                  columns and products in one kernel.
+// pwa_columns_f64  per-event partial-wave columns F_k, and
+// pwa_gram_f64     the same sums from them, for models whose event tile does
+//                  not fit in shared memory.
 #pragma once
 
 #ifndef PWA_TPB
@@ -257,6 +260,178 @@ extern "C" __global__ void pwa_sum_rows(const double* __restrict__ in, int nrows
     s = warp_sum(s);
     if (lane == 0) out[j] = s;
   }
+}
+
+// sqrt(|P_l(z0)|) of every vertex (the sp argument of model_cols) into
+// shared memory, one value per thread: constant indices only (an index that
+// depends on the thread would copy the constant block to local memory), one
+// square root for all threads.  Ends without a barrier.
+__device__ __forceinline__ void stage_sp(const Consts& C, double* s_sp) {
+#pragma unroll 1
+  for (int j0 = 0; j0 < PWA_NSP; j0 += PWA_TPB) {
+    double v = 0.0;
+#pragma unroll
+    for (int j = 0; j < PWA_NSP; ++j)
+      if (j == j0 + (int)threadIdx.x) v = C.v[pwa_sp_const[j]];
+    if (j0 + (int)threadIdx.x < PWA_NSP) s_sp[j0 + threadIdx.x] = sqrt(fabs(v));
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Gram matrix of the MC set straight from the events: columns and their
+// weighted products in one kernel, nothing but block sums written.
+//
+// A block forms the columns of PWA_TPB events into shared memory, X[r][c]
+// with r = (helicity o, event) and c = 2k, 2k + 1 = Re, Im F_k,o, then adds
+// G = X^T W X (real, 2K x 2K, lower 8 x 8 tiles) with FP64 matrix
+// instructions, mma.m8n8k4: a lane's value of the A operand (column
+// 8 bi + lane / 4 of row r = lane % 4) and of the B operand are the same
+// shared-memory word, so one load per 8 columns and 4 rows feeds every
+// tile; rows of GM_LD = CP + 4 doubles put the 16 lanes of a load phase in
+// distinct banks.  Re M_kl = G[2k][2l] + G[2k+1][2l+1], Im M_kl =
+// G[2k][2l+1] - G[2k+1][2l].
+// Bound: the FP64 pipe (columns and products) at three blocks per SM
+// (68 KB, 164 registers, four-body).  The two-kernel form it replaces
+// (columns to memory, 480 B per four-body event, then one thread per (k, l)
+// reading two operands per product from shared memory, and a 256 MB buffer
+// allocated and freed per call): a whole fit set-up, column cache of 3e5 and
+// Gram of 1.2e6 four-body events, took 5.1 ms and takes 0.60 ms.  Models
+// whose tile exceeds GM_MAX_BYTES (many helicities x columns: two blocks
+// would not fit on an SM) keep that form.
+#define GM_CP ((2 * PWA_NCOL + 7) / 8 * 8)
+#define GM_LD (GM_CP + 4)
+#define GM_NT (GM_CP / 8)
+#define GM_TT (GM_NT * (GM_NT + 1) / 2)
+#define GM_NW (PWA_TPB / 32)
+#define GM_MAX_BYTES (104 * 1024)
+#define GM_BYTES (PWA_NOUT * PWA_TPB * GM_LD * 8)
+#define PWA_GRAM_FUSED (GM_BYTES <= GM_MAX_BYTES && GM_TT <= 12 * GM_NW)
+// few tiles (at most 10): every warp holds all of them and takes every
+// GM_NW-th group of four rows; more: the warps split the tiles
+#define GM_ROWSPLIT (GM_TT <= 10)
+
+__device__ __forceinline__ void mma_f64(double& d0, double& d1, double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+               : "+d"(d0), "+d"(d1)
+               : "d"(a), "d"(b));
+}
+
+struct GramSink {  // rows of X of one event
+  double* x;
+  __device__ __forceinline__ void set(int k, int o, int, double re, double im) {
+    *reinterpret_cast<double2*>(x + o * (PWA_TPB * GM_LD) + 2 * k) = make_double2(re, im);
+  }
+  __device__ __forceinline__ void add(int k, int o, int, double re, double im) {
+    double2* p = reinterpret_cast<double2*>(x + o * (PWA_TPB * GM_LD) + 2 * k);
+    *p = make_double2(p->x + re, p->y + im);
+  }
+};
+
+// tiles [T0, T1) of the lower triangle (row by row) over rows 4 s .. 4 s + 3
+// of X, s = s0, s0 + ds, ...
+template <int T0, int T1>
+__device__ __forceinline__ void gram_tiles(const double* __restrict__ X,
+                                           const double* __restrict__ sw, int s0, int ds, int lane,
+                                           double (&acc)[2 * (T1 - T0)]) {
+  const double* xp = X + (lane & 3) * GM_LD + (lane >> 2);
+#pragma unroll 2
+  for (int s = s0; s < PWA_NOUT * PWA_TPB / 4; s += ds) {
+    const double w = sw[(4 * s + (lane & 3)) % PWA_TPB];
+    double x[GM_NT];
+#pragma unroll
+    for (int b = 0; b < GM_NT; ++b) x[b] = xp[4 * s * GM_LD + 8 * b];
+    int t = 0;
+#pragma unroll
+    for (int bi = 0; bi < GM_NT; ++bi) {
+      const double a = w * x[bi];
+#pragma unroll
+      for (int bj = 0; bj <= bi; ++bj, ++t)
+        if (t >= T0 && t < T1) mma_f64(acc[2 * (t - T0)], acc[2 * (t - T0) + 1], a, x[bj]);
+    }
+  }
+}
+
+#if PWA_GRAM_FUSED
+#define GM_PER ((GM_TT + GM_NW - 1) / GM_NW)
+template <int W>
+__device__ __forceinline__ void gram_warp(const double* X, const double* sw, int warp, int lane,
+                                          double (&acc)[2 * (GM_ROWSPLIT ? GM_TT : GM_PER)]) {
+#if GM_ROWSPLIT
+  gram_tiles<0, GM_TT>(X, sw, warp, GM_NW, lane, acc);
+#else
+  if constexpr (W < GM_NW) {
+    if (warp == W) {
+      constexpr int T0 = W * GM_PER < GM_TT ? W * GM_PER : GM_TT;
+      gram_tiles<T0, T0 + GM_PER>(X, sw, 0, 1, lane, acc);
+    } else {
+      gram_warp<W + 1>(X, sw, warp, lane, acc);
+    }
+  }
+#endif
+}
+#endif
+
+// blocks walk the tiles of PWA_TPB events of [beg, end); partials: GM_TT * 64
+// doubles per block (tile, lane, 2), summed by pwa_sum_rows
+extern "C" __global__ void __launch_bounds__(PWA_TPB)
+    pwa_gram_fused(const Consts C, const double* __restrict__ XA, const double* __restrict__ XM,
+                   const double* __restrict__ W, long long beg, long long end, long long ld,
+                   double* __restrict__ partials) {
+#if PWA_GRAM_FUSED
+  extern __shared__ __align__(16) double gm_x[];
+  __shared__ double s_w[PWA_TPB];
+  __shared__ double s_sp[PWA_NSP];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  // the padding columns and the pairs without a value stay zero
+  for (int j = tid; j < PWA_NOUT * PWA_TPB * GM_LD; j += PWA_TPB) gm_x[j] = 0.0;
+  stage_sp(C, s_sp);
+  __syncthreads();
+  double acc[2 * (GM_ROWSPLIT ? GM_TT : GM_PER)];
+#pragma unroll
+  for (int j = 0; j < 2 * (GM_ROWSPLIT ? GM_TT : GM_PER); ++j) acc[j] = 0.0;
+  double* row = gm_x + tid * GM_LD;
+  for (long long t0 = beg + (long long)blockIdx.x * PWA_TPB; t0 < end;
+       t0 += (long long)gridDim.x * PWA_TPB) {
+    const long long i = t0 + tid;
+    if (i < end) {
+      s_w[tid] = __ldg(W + i);
+      GramSink sink{row};
+      model_cols<true>(C, s_sp, XA, XM, ld, i, sink);
+    } else {
+      s_w[tid] = 0.0;
+      for (int o = 0; o < PWA_NOUT; ++o)
+        for (int c = 0; c < 2 * PWA_NCOL; ++c) row[o * (PWA_TPB * GM_LD) + c] = 0.0;
+    }
+    __syncthreads();
+    gram_warp<0>(gm_x, s_w, warp, lane, acc);
+    __syncthreads();
+  }
+  double* out = partials + (long long)blockIdx.x * (GM_TT * 64);
+#if GM_ROWSPLIT
+  {
+    // the warps' sums of each tile, in warp order (GM_TT * 64 <= 640 doubles)
+    for (int w2 = 0; w2 < GM_NW; ++w2) {
+      if (warp == w2) {
+#pragma unroll
+        for (int j = 0; j < 2 * GM_TT; ++j) {
+          double* p = gm_x + (j >> 1) * 64 + 2 * lane + (j & 1);
+          *p = w2 ? *p + acc[j] : acc[j];
+        }
+      }
+      __syncthreads();
+    }
+    for (int j = tid; j < GM_TT * 64; j += PWA_TPB) out[j] = gm_x[j];
+  }
+#else
+  {
+#pragma unroll
+    for (int j = 0; j < 2 * GM_PER; ++j) {
+      const int t = warp * GM_PER + (j >> 1);
+      if (t < GM_TT) out[t * 64 + 2 * lane + (j & 1)] = acc[j];
+    }
+  }
+#endif
+#endif
 }
 
 // ---------------------------------------------------------------------------
@@ -572,26 +747,54 @@ extern "C" __global__ void pwa_to_f32(const double* __restrict__ in, float* __re
 // A tile is one contiguous block, so one bulk copy moves it to shared memory.
 // Values are computed in FP64 and rounded to FP32 once per stored value
 // (unbiased per-event rounding, no systematic bias in sums over events).
+// One pass: each pair goes to memory as it is formed (no array of all columns
+// in registers).  With swaps the passes' FP64 values are summed first.
+struct CacheSink {
+  float2* d;  // pair 0 of the event
+  __device__ __forceinline__ void set(int, int, int j, double re, double im) {
+    d[j * PWA_TPB] = make_float2((float)re, (float)im);
+  }
+  __device__ __forceinline__ void add(int, int, int, double, double) {}
+};
+template <bool SHAPES>
+__device__ __forceinline__ void cache_event(const Consts& C, const double* sp,
+                                            const double* __restrict__ XA,
+                                            const double* __restrict__ XM, long long ld,
+                                            long long i, float2* __restrict__ d) {
+#if PWA_NPASS == 1
+  CacheSink s{d};
+  if constexpr (SHAPES) model_cols<true>(C, sp, XA, XM, ld, i, s);
+  else model_cols_ns<true>(C, sp, XA, XM, ld, i, s);
+#else
+  cpx<double> F[PWA_NCOL * PWA_NOUT];
+  DenseColumns s{F};
+  if constexpr (SHAPES) model_cols<true>(C, sp, XA, XM, ld, i, s);
+  else model_cols_ns<true>(C, sp, XA, XM, ld, i, s);
+#pragma unroll
+  for (int j = 0; j < PWA_NF; ++j) {
+    const cpx<double> v = F[pwa_fk[j] * PWA_NOUT + pwa_fo[j]];
+    d[j * PWA_TPB] = make_float2((float)v.re, (float)v.im);
+  }
+#endif
+}
 extern "C" __global__ void __launch_bounds__(PWA_TPB)
     pwa_cache_f32(const Consts C, const double* __restrict__ XA, const double* __restrict__ XM,
                   const double* __restrict__ W, long long n, long long ntiles, long long ld,
                   float2* __restrict__ Fc, double* __restrict__ Wc) {
+  __shared__ double s_sp[PWA_NSP];
+  stage_sp(C, s_sp);
+  __syncthreads();
   const long long total = ntiles * PWA_TPB;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
     const long long t = i / PWA_TPB, e = i % PWA_TPB;
+    float2* d = Fc + t * PWA_NF * PWA_TPB + e;
     if (i < n) {
-      cpx<double> F[PWA_NCOL * PWA_NOUT];
-      model_columns<double>(C, XA, XM, ld, i, F);
-#pragma unroll
-      for (int j = 0; j < PWA_NF; ++j) {
-        const cpx<double> v = F[pwa_fk[j] * PWA_NOUT + pwa_fo[j]];
-        Fc[(t * PWA_NF + j) * PWA_TPB + e] = make_float2((float)v.re, (float)v.im);
-      }
+      cache_event<true>(C, s_sp, XA, XM, ld, i, d);
       Wc[i] = W[i];
     } else {
 #pragma unroll
-      for (int j = 0; j < PWA_NF; ++j) Fc[(t * PWA_NF + j) * PWA_TPB + e] = make_float2(0.f, 0.f);
+      for (int j = 0; j < PWA_NF; ++j) d[j * PWA_TPB] = make_float2(0.f, 0.f);
       Wc[i] = 0.0;
     }
   }
@@ -615,21 +818,19 @@ extern "C" __global__ void __launch_bounds__(PWA_TPB)
 extern "C" __global__ void __launch_bounds__(PWA_TPB)
     pwa_cache_ns_f32(const Consts C, const double* __restrict__ XA, const double* __restrict__ XM,
                      long long n, long long ntiles, long long ld, float2* __restrict__ Fc) {
+  __shared__ double s_sp[PWA_NSP];
+  stage_sp(C, s_sp);
+  __syncthreads();
   const long long total = ntiles * PWA_TPB;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
     const long long t = i / PWA_TPB, e = i % PWA_TPB;
+    float2* d = Fc + t * PWA_NF * PWA_TPB + e;
     if (i < n) {
-      cpx<double> F[PWA_NCOL * PWA_NOUT];
-      model_columns_ns<double>(C, XA, XM, ld, i, F);
-#pragma unroll
-      for (int j = 0; j < PWA_NF; ++j) {
-        const cpx<double> v = F[pwa_fk[j] * PWA_NOUT + pwa_fo[j]];
-        Fc[(t * PWA_NF + j) * PWA_TPB + e] = make_float2((float)v.re, (float)v.im);
-      }
+      cache_event<false>(C, s_sp, XA, XM, ld, i, d);
     } else {
 #pragma unroll
-      for (int j = 0; j < PWA_NF; ++j) Fc[(t * PWA_NF + j) * PWA_TPB + e] = make_float2(0.f, 0.f);
+      for (int j = 0; j < PWA_NF; ++j) d[j * PWA_TPB] = make_float2(0.f, 0.f);
     }
   }
 }

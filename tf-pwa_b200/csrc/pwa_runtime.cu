@@ -41,7 +41,7 @@ struct Kernels {
                eval_cached_wide = nullptr, eval_cached_tma = nullptr, eval_multi = nullptr,
                gram_colmax = nullptr, gram_tc = nullptr, wait_check = nullptr,
                fma_f64 = nullptr, fma_f32 = nullptr, eval_points = nullptr, reduce_multi = nullptr,
-               hess_cached = nullptr, cache_ns_f32 = nullptr, eval_shapecache = nullptr,
+               gram_fused = nullptr, hess_cached = nullptr, cache_ns_f32 = nullptr, eval_shapecache = nullptr,
                fields_from_p4 = nullptr, toy_select = nullptr, toy_fields = nullptr;
 };
 
@@ -438,6 +438,7 @@ int pwa_plan_create(const char* src, size_t src_len, int n_mass, int n_angle, in
             {"pwa_eval_cached_wide", &h->k.eval_cached_wide},
             {"pwa_eval_cached_tma", &h->k.eval_cached_tma},
             {"pwa_gram_colmax", &h->k.gram_colmax},
+            {"pwa_gram_fused", &h->k.gram_fused},
             {"pwa_gram_tc", &h->k.gram_tc},
             {"pwa_wait_check", &h->k.wait_check},
             {"pwa_fma_peak_f64", &h->k.fma_f64},
@@ -851,12 +852,83 @@ int pwa_set_gram_method(pwa_plan* h, int method) {
   return PWA_OK;
 }
 
+namespace {
+// Shared memory of one block of pwa_gram_fused and its count of 8 x 8 tiles
+// (GM_* of the device header); 0 bytes where the kernel is compiled empty.
+size_t gram_fused_bytes(const pwa_plan* h, int* tiles) {
+  const int cp = (2 * h->ncol + 7) / 8 * 8, nt = cp / 8;
+  *tiles = nt * (nt + 1) / 2;
+  const size_t bytes = (size_t)h->nout * h->tpb * (cp + 4) * sizeof(double);
+  return bytes <= 104 * 1024 && *tiles <= 12 * (h->tpb / 32) ? bytes : 0;
+}
+
+// The Gram matrix in one pass over the MC events (columns and products in
+// one kernel; block sums in the plan's workspace, summed in block order).
+int gram_fused(pwa_plan* h, const std::vector<double>& cbuf, size_t smem, int tiles,
+               cudaStream_t s, std::vector<double>* acc) {
+  CU(cudaFuncSetAttribute((const void*)h->k.gram_fused,
+                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  int per_sm = 0;
+  CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)h->k.gram_fused, h->tpb,
+                                                   smem));
+  if (per_sm < 1) per_sm = 1;
+  const long long want = (long long)per_sm * h->sms, need = (h->n_mc + h->tpb - 1) / h->tpb;
+  int nrows = (int)(want < need ? want : need), ncols = tiles * 64;
+  int rc = ensure_partials(h, ((long long)nrows + 1) * ncols);
+  if (rc) return rc;
+  long long beg = h->n_data, end = h->n_data + h->n_mc, ld = h->ld;
+  void* a1[] = {(void*)cbuf.data(), &h->xa, &h->xm, &h->w, &beg, &end, &ld, &h->partials};
+  cudaError_t e = cudaLaunchKernel((const void*)h->k.gram_fused, dim3(nrows), dim3(h->tpb), a1,
+                                   smem, s);
+  if (e != cudaSuccess)
+    return set_err(h, PWA_ERR_CUDA, std::string("gram kernel launch: ") + cudaGetErrorString(e));
+  double* gsum = h->partials + (long long)nrows * ncols;
+  void* a2[] = {&h->partials, &nrows, &ncols, &gsum};
+  rc = launch(h, h->k.sum_rows, dim3((ncols + 7) / 8), dim3(256), a2, s);
+  if (rc) return rc;
+  std::vector<double> t((size_t)ncols);
+  CU(cudaMemcpyAsync(t.data(), gsum, sizeof(double) * ncols, cudaMemcpyDeviceToHost, s));
+  CU(cudaStreamSynchronize(s));
+  // real symmetric G from its lower tiles: lane l holds row l / 4, columns
+  // 2 (l % 4), 2 (l % 4) + 1 of an 8 x 8 tile
+  const int K = h->ncol, cp = (2 * K + 7) / 8 * 8;
+  std::vector<double> G((size_t)cp * cp, 0.0);
+  const double* q = t.data();
+  for (int bi = 0; bi < cp / 8; ++bi)
+    for (int bj = 0; bj <= bi; ++bj, q += 64)
+      for (int l = 0; l < 32; ++l)
+        for (int u = 0; u < 2; ++u) {
+          const int c = 8 * bi + l / 4, d = 8 * bj + 2 * (l % 4) + u;
+          if (c >= d) G[(size_t)c * cp + d] = G[(size_t)d * cp + c] = q[2 * l + u];
+        }
+  for (int k = 0; k < K; ++k)
+    for (int l = 0; l < K; ++l) {
+      const double* r0 = &G[(size_t)(2 * k) * cp + 2 * l];
+      const double* r1 = r0 + cp;
+      (*acc)[2 * ((size_t)k * K + l)] = r0[0] + r1[1];
+      (*acc)[2 * ((size_t)k * K + l) + 1] = r0[1] - r1[0];
+    }
+  return PWA_OK;
+}
+}  // namespace
+
 int pwa_build_gram(pwa_plan* h, const double* consts, void* stream, double* out) {
   if (!h) return PWA_ERR_ARG;
   if (!h->w || h->n_mc <= 0) return set_err(h, PWA_ERR_STATE, "no MC events uploaded");
   if (!consts) return set_err(h, PWA_ERR_ARG, "invalid gram arguments");
   cudaStream_t s = (cudaStream_t)stream;
   const bool tc = h->gram_method == 1 && 2 * h->ncol <= 64;
+  int tiles = 0;
+  const size_t fused = gram_fused_bytes(h, &tiles);
+  if (!tc && fused) {
+    std::vector<double> acc(2 * (size_t)h->ncol * h->ncol);
+    const int rc = gram_fused(h, consts_block(h, consts), fused, tiles, s, &acc);
+    if (rc) return rc;
+    h->gram = acc;
+    h->gram_valid = true;
+    if (out) std::memcpy(out, acc.data(), sizeof(double) * acc.size());
+    return PWA_OK;
+  }
   std::vector<double> cbuf = consts_block(h, consts);
   const long long row = 2LL * h->ncol * h->nout;
   // chunked: columns of at most `chunk` events at a time
