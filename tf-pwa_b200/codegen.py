@@ -952,6 +952,9 @@ class ModelCode:
         L.append("__device__ constexpr int pwa_sres_chain[PWA_NSRES > 0 ? PWA_NSRES : 1][PWA_NCHAIN] = {" +
                  (", ".join("{" + r + "}" for r in rows) if rows else "{" + ", ".join(["0"] * nch) + "}") + "};")
         L.append(self._pdf_source())
+        # sum |A|^2 linear in fixed column couplings: the FP64 evaluation may
+        # work from the columns (no density matrix, no per-charge totals)
+        L.append(f"#define PWA_COLS_EVAL {0 if self.pol_names or self.cp_chains else 1}")
         fl = sorted(self._fset)
         L.append(f"#define PWA_NF {self.nf}")
         # blocks per SM of the plain FP64 kernels: 4 where the accumulators

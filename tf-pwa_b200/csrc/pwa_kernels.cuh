@@ -1037,6 +1037,167 @@ extern "C" __global__ void __launch_bounds__(PWA_TPB, PWA_SC_MINB)
   publish_result(ticket, NA2, out, seq);
 }
 
+// Plain FP64 evaluation from the columns, where no mass or width is free (no
+// lineshape sums are asked for).  pwa_eval_f64 forms each event's amplitude,
+// then forms every angular factor, barrier and lineshape again for the
+// adjoint, with all accumulators in registers; here each column is formed
+// once.
+//
+// A block takes PWA_TPB events at a time.  (1) Each thread forms its event's
+// columns: a value goes to shared memory and into A_o = sum c_k F_k,o at
+// once; then f, clip_log and the seed fac conj(A_o), also to shared memory.
+// (2) Warp v takes the columns k = v, v + 4, ...: its lanes walk the block's
+// events and add the seed times F_k,o to two sums per column, so a thread
+// holds 2 K / 4 accumulators instead of 1 + 2 K + 2 resonances (four-body:
+// 16 instead of 85, which spilled).
+// Ends with the ordered two-level reduction of pwa_eval_shapecache: row
+// halves for data and MC blocks, result in mapped memory, one launch.
+// Bound: the FP64 pipe and its latency at three blocks per SM (shared
+// memory).  Measured against pwa_eval_f64 and its reduce launch, whole
+// evaluations: four-body 1e6 events 237 vs 1098 us, Lambda_c 2.1e6 379 vs
+// 655 us, D -> K pi pi 1.1e5 23 vs 29 us.
+// Models with a density matrix, per-charge totals or more pairs than fit
+// (EC_MAX_BYTES) keep pwa_eval_f64, as do evaluations with free masses or
+// widths, which need the lineshape sums.
+#define EC_NW (PWA_TPB / 32)
+#define EC_KW ((PWA_NCOL + EC_NW - 1) / EC_NW)
+#define EC_MAX_BYTES (110 * 1024)
+#define EC_BYTES ((PWA_NF + PWA_NOUT) * PWA_TPB * 16)
+#define PWA_EVAL_COLS (PWA_COLS_EVAL && EC_BYTES <= EC_MAX_BYTES)
+#ifndef EC_MINB
+#define EC_MINB (EC_BYTES <= 74 * 1024 ? 3 : 2)
+#endif
+
+struct EvalSink {
+  const Consts& C;
+  double2* s;  // pair 0 of the thread's event
+  double (&ar)[PWA_NOUT];
+  double (&ai)[PWA_NOUT];
+  __device__ __forceinline__ void amp(int k, int o, double re, double im) {
+    ar[o] = fma(C.v[2 * k], re, fma(-C.v[2 * k + 1], im, ar[o]));
+    ai[o] = fma(C.v[2 * k], im, fma(C.v[2 * k + 1], re, ai[o]));
+  }
+  __device__ __forceinline__ void set(int k, int o, int j, double re, double im) {
+    s[j * PWA_TPB] = make_double2(re, im);
+    amp(k, o, re, im);
+  }
+  __device__ __forceinline__ void add(int k, int o, int j, double re, double im) {
+    const double2 v = s[j * PWA_TPB];
+    s[j * PWA_TPB] = make_double2(v.x + re, v.y + im);
+    amp(k, o, re, im);
+  }
+};
+
+// sums of columns V, V + EC_NW, ... over the block's events (warp V)
+template <int V>
+__device__ __forceinline__ void eval_cols_adjoint(const double2* sF, const double2* sA, int warp,
+                                                  int lane, double (&acc)[2 * EC_KW]) {
+  if constexpr (V < EC_NW) {
+    if (warp == V) {
+#pragma unroll 1
+      for (int e = lane; e < PWA_TPB; e += 32) {
+        double2 a[PWA_NOUT];
+#pragma unroll
+        for (int o = 0; o < PWA_NOUT; ++o) a[o] = sA[o * PWA_TPB + e];
+#pragma unroll
+        for (int j = 0; j < PWA_NF; ++j) {
+          if (pwa_fk[j] % EC_NW != V) continue;
+          const int q = pwa_fk[j] / EC_NW;
+          const double2 v = sF[j * PWA_TPB + e], b = a[pwa_fo[j]];
+          acc[2 * q] = fma(b.x, v.x, fma(-b.y, v.y, acc[2 * q]));
+          acc[2 * q + 1] = fma(b.x, v.y, fma(b.y, v.x, acc[2 * q + 1]));
+        }
+      }
+    } else {
+      eval_cols_adjoint<V + 1>(sF, sA, warp, lane, acc);
+    }
+  }
+}
+
+extern "C" __global__ void __launch_bounds__(PWA_TPB, EC_MINB)
+    pwa_eval_cols(const Consts C, const double* __restrict__ XA, const double* __restrict__ XM,
+                  const double* __restrict__ W, long long n_data, long long n_all, long long ld,
+                  int blocks_data, double* __restrict__ partials,
+                  unsigned int* __restrict__ ticket, double* __restrict__ out, double seq) {
+#if PWA_EVAL_COLS
+  extern __shared__ __align__(16) double2 ec_smem[];
+  double2* sF = ec_smem;                      // [PWA_NF][PWA_TPB]
+  double2* sA = ec_smem + PWA_NF * PWA_TPB;   // [PWA_NOUT][PWA_TPB]
+  __shared__ double s_sp[PWA_NSP];
+  __shared__ double s_sum[1 + 2 * PWA_NCOL], s_s0[EC_NW];
+  __shared__ int s_last;
+  const bool is_data = (int)blockIdx.x < blocks_data;
+  const long long end = is_data ? n_data : n_all;
+  const int nb = is_data ? blocks_data : (int)gridDim.x - blocks_data;
+  const int b = is_data ? (int)blockIdx.x : (int)blockIdx.x - blocks_data;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  stage_sp(C, s_sp);
+  __syncthreads();
+  double acc0 = 0.0, acc[2 * EC_KW];
+#pragma unroll
+  for (int j = 0; j < 2 * EC_KW; ++j) acc[j] = 0.0;
+  for (long long t0 = (is_data ? 0 : n_data) + (long long)b * PWA_TPB; t0 < end;
+       t0 += (long long)nb * PWA_TPB) {
+    const long long i = t0 + tid;
+    if (i < end) {
+      double ar[PWA_NOUT], ai[PWA_NOUT];
+#pragma unroll
+      for (int o = 0; o < PWA_NOUT; ++o) ar[o] = ai[o] = 0.0;
+      EvalSink sink{C, sF + tid, ar, ai};
+      model_cols<true>(C, s_sp, XA, XM, ld, i, sink);
+      double f = 0.0;
+#pragma unroll
+      for (int o = 0; o < PWA_NOUT; ++o) f = fma(ar[o], ar[o], fma(ai[o], ai[o], f));
+      const double w = __ldg(W + i);
+      double fac = w;
+      if (is_data) {
+        double dl;
+        const double cl = clip_log(f, &dl);
+        acc0 = fma(w, cl, acc0);
+        fac = w * dl;
+      } else {
+        acc0 = fma(w, f, acc0);
+      }
+#pragma unroll
+      for (int o = 0; o < PWA_NOUT; ++o)
+        sA[o * PWA_TPB + tid] = make_double2(fac * ar[o], -fac * ai[o]);
+    } else {  // past the end of the set: nothing to add
+      for (int j = 0; j < PWA_NF + PWA_NOUT; ++j) sF[j * PWA_TPB + tid] = make_double2(0.0, 0.0);
+    }
+    __syncthreads();
+    eval_cols_adjoint<0>(sF, sA, warp, lane, acc);
+    __syncthreads();
+  }
+  acc0 = warp_sum(acc0);
+  if (lane == 0) s_s0[warp] = acc0;
+#pragma unroll
+  for (int q = 0; q < EC_KW; ++q) {
+    const double re = warp_sum(acc[2 * q]), im = warp_sum(acc[2 * q + 1]);
+    const int k = warp + EC_NW * q;
+    if (lane == 0 && k < PWA_NCOL) {
+      s_sum[1 + 2 * k] = re;
+      s_sum[2 + 2 * k] = im;
+    }
+  }
+  __syncthreads();
+  if (tid == 0) {
+    double s = 0.0;
+    for (int v = 0; v < EC_NW; ++v) s += s_s0[v];
+    s_sum[0] = s;
+  }
+  __syncthreads();
+  constexpr int NA2 = 2 * PWA_NACC;
+  for (int j = tid; j < NA2; j += PWA_TPB) {
+    const int jj = j - (is_data ? 0 : PWA_NACC);
+    partials[(long long)blockIdx.x * NA2 + j] = jj >= 0 && jj < 1 + 2 * PWA_NCOL ? s_sum[jj] : 0.0;
+  }
+  __threadfence();
+  __syncthreads();
+  if (!grouped_sum(partials, ticket, NA2, out, &s_last)) return;
+  publish_result(ticket, NA2, out, seq);
+#endif
+}
+
 struct CCoup {
   double v[2 * PWA_NCOL];  // column couplings c_k, (re, im) pairs
 };

@@ -41,7 +41,7 @@ struct Kernels {
                eval_cached_wide = nullptr, eval_cached_tma = nullptr, eval_multi = nullptr,
                gram_colmax = nullptr, gram_tc = nullptr, wait_check = nullptr,
                fma_f64 = nullptr, fma_f32 = nullptr, eval_points = nullptr, reduce_multi = nullptr,
-               gram_fused = nullptr, hess_cached = nullptr, cache_ns_f32 = nullptr, eval_shapecache = nullptr,
+               gram_fused = nullptr, eval_cols = nullptr, hess_cached = nullptr, cache_ns_f32 = nullptr, eval_shapecache = nullptr,
                fields_from_p4 = nullptr, toy_select = nullptr, toy_fields = nullptr;
 };
 
@@ -125,6 +125,9 @@ struct pwa_plan {
   int sc_stages = 0;  // PWA_SC_STAGES of the model source
   int sc_smem = 0;    // dynamic shared memory of pwa_eval_shapecache
   bool shape_cache_ok = false;  // the model's columns factorise (PWA_SHAPE_CACHE_OK 1)
+  // plain FP64 evaluation from the columns (pwa_eval_cols): shared memory of
+  // a block (0: the model keeps pwa_eval_f64) and its grid (0: not set up)
+  int ec_smem = 0, ec_blocks = 0, ec_blocks_data = 0;
   double* d_hsum = nullptr;
   // parameter layout for the C-side chain rule
   int n_vars = 0, n_coup = 0, nfac = 0, n_train = 0;
@@ -389,6 +392,10 @@ int pwa_plan_create(const char* src, size_t src_len, int n_mass, int n_angle, in
     const size_t at = text.find(key);
     h->sc_stages = at == std::string::npos ? 0 : std::atoi(text.c_str() + at + key.size());
   }
+  // EC_BYTES, EC_MAX_BYTES of the device header
+  if (std::string(src, src_len).find("#define PWA_COLS_EVAL 1") != std::string::npos &&
+      (nf + nout) * tpb * 16 <= 110 * 1024)
+    h->ec_smem = (nf + nout) * tpb * 16;
   h->n_angle = n_angle;
   h->ncol = ncol;
   h->nout = nout;
@@ -439,6 +446,7 @@ int pwa_plan_create(const char* src, size_t src_len, int n_mass, int n_angle, in
             {"pwa_eval_cached_tma", &h->k.eval_cached_tma},
             {"pwa_gram_colmax", &h->k.gram_colmax},
             {"pwa_gram_fused", &h->k.gram_fused},
+            {"pwa_eval_cols", &h->k.eval_cols},
             {"pwa_gram_tc", &h->k.gram_tc},
             {"pwa_wait_check", &h->k.wait_check},
             {"pwa_fma_peak_f64", &h->k.fma_f64},
@@ -524,6 +532,7 @@ int pwa_upload_events(pwa_plan* h, const double* xm, const double* xa, const dou
   h->n_mc = n_mc;
   h->fcache_n = 0;
   h->scache_n = 0;  // the floating-shape column cache belongs to the old events
+  h->ec_blocks = 0;
   h->gram_valid = false;
   const cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
   if (h->n_mass)
@@ -619,6 +628,64 @@ int wait_mapped_sums(pwa_plan* h, cudaStream_t s) {
     return set_err(h, PWA_ERR_CUDA, "evaluation did not complete (stale result)");
   }
   return PWA_OK;
+}
+}  // namespace
+
+namespace {
+// Blocks for td data and tm MC tiles on at most `most` blocks: the fewest
+// tiles r per block for which both sets' blocks fit, so that no block takes
+// one tile more than the others (a split in proportion to the events rounds
+// one set's share up and leaves its blocks a whole tile behind).
+void split_tiles(long long td, long long tm, long long most, int* blocks, int* data) {
+  long long r = (td + tm + most - 1) / most;
+  if (r < 1) r = 1;
+  while ((td + r - 1) / r + (tm + r - 1) / r > most) ++r;
+  *data = (int)((td + r - 1) / r);
+  *blocks = (int)(*data + (tm + r - 1) / r);
+}
+
+// Plain FP64 sums without the lineshape sums (pwa_eval_cols).
+int eval_cols(pwa_plan* h, const double* consts, cudaStream_t s, double* out) {
+  if (!h->w) return set_err(h, PWA_ERR_STATE, "no events uploaded");
+  if (h->ec_blocks == 0) {
+    CU(cudaFuncSetAttribute((const void*)h->k.eval_cols,
+                            cudaFuncAttributeMaxDynamicSharedMemorySize, h->ec_smem));
+    int per_sm = 0;
+    CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)h->k.eval_cols, h->tpb,
+                                                     h->ec_smem));
+    if (per_sm < 1) per_sm = 1;
+    const long long t = h->tpb;
+    int nb = 0, bd = 0;
+    split_tiles((h->n_data + t - 1) / t, (h->n_mc + t - 1) / t, (long long)per_sm * h->sms, &nb,
+                &bd);
+    const int rc = ensure_partials(h, (long long)(nb + (nb + 15) / 16) * 2 * h->nacc);
+    if (rc) return rc;
+    h->ec_blocks_data = bd;
+    h->ec_blocks = nb;
+  }
+  std::vector<double> cbuf = consts_block(h, consts);
+  long long nd = h->n_data, na = h->n_data + h->n_mc, ld = h->ld;
+  h->seq += 1.0;
+  double seq = h->seq;
+  void* args[] = {cbuf.data(), &h->xa, &h->xm, &h->w, &nd, &na, &ld, &h->ec_blocks_data,
+                  &h->partials, &h->ticket, &h->d_map_sc, &seq};
+  cudaError_t e = cudaLaunchKernel((const void*)h->k.eval_cols, dim3(h->ec_blocks), dim3(h->tpb),
+                                   args, (size_t)h->ec_smem, s);
+  if (e != cudaSuccess)
+    return set_err(h, PWA_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e));
+  int rc = wait_mapped_sums(h, s);
+  if (rc) return rc;
+  const volatile double* m = h->h_map_sc;
+  for (int j = 0; j < 2 * h->nacc; ++j) out[j] = m[j];
+  return PWA_OK;
+}
+
+// Whether no trainable variable takes a derivative through the kernels'
+// lineshape sums.
+bool no_shape_sums(const pwa_hostprog& p) {
+  for (int s : p.t_sel)
+    if (s >= 0) return false;
+  return true;
 }
 }  // namespace
 
@@ -2144,6 +2211,8 @@ int pwa_pieces_vars(pwa_plan* h, const double* vars, int form, double sw, double
       // so this point recomputes them (FP32 amplitudes)
       rc = pwa_eval(h, C.data(), PWA_MIXED_F32, 1, stream, sums.data());
     }
+  } else if (form == PWA_FORM_PLAIN_F64 && h->ec_smem > 0 && no_shape_sums(*p)) {
+    rc = eval_cols(h, C.data(), (cudaStream_t)stream, sums.data());
   } else {
     rc = pwa_eval(h, C.data(), form == PWA_FORM_PLAIN_F64 ? PWA_PLAIN_F64 : PWA_MIXED_F32, 1,
                   stream, sums.data());
