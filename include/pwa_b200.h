@@ -121,6 +121,12 @@ int pwa_eval_pdf(pwa_plan* h, const double* consts, int precision, long long beg
  * field in plan order with stride ld_out.  Enqueued on `stream`. */
 int pwa_fields_from_p4(pwa_plan* h, const double* p4, long long n, long long ld_in, double* out,
                        long long ld_out, void* stream);
+/* The same from momenta of any layout: component c of final f of event i is
+ * p4[i stride_event + f stride_final + c stride_comp] (strides in doubles,
+ * >= 0; an (N, n_final, 4) array has 4 n_final, 4, 1). */
+int pwa_fields_from_strided(pwa_plan* h, const double* p4, long long n, long long stride_event,
+                            long long stride_final, long long stride_comp, double* out,
+                            long long ld_out, void* stream);
 
 /* Toy / MC generation on the device (tf_pwa/phasespace.py:31-254 flat phase
  * space; tf_pwa/applications.py:394-487 accept-reject on sum |A|^2).

@@ -13,6 +13,12 @@
 //   * clip_log ....................................... tf_pwa/model/model.py:283-292
 #pragma once
 
+#ifdef __CUDACC__
+#define PWA_NOINLINE __noinline__
+#else
+#define PWA_NOINLINE inline
+#endif
+
 // ---------------------------------------------------------------- complex
 template <typename R>
 struct cpx {
@@ -418,23 +424,83 @@ __device__ __forceinline__ void kin_angle_zx_z_getx(V3 z1, V3 x1, V3 z2, double*
   *beta = kin_angle_from(u_z2, u_z1, u_xr);
   *x2 = kin_cross_unit(u_yr, u_z2);
 }
-// alpha folded into [bias, bias + 2 pi)
-__device__ __forceinline__ double kin_fold(double a, double bias) {
-  const double tp = 2.0 * 3.141592653589793, x = a - bias;
-  return x - tp * floor(x / tp) + bias;
-}
-// `o` boosted into the rest frame of `p`
-__device__ __forceinline__ LV kin_rest_vector(LV p, LV o) {
-  const V3 pb = {-p.x / p.t, -p.y / p.t, -p.z / p.t};
-  const double beta2 = v3_dot(pb, pb);
-  const double gamma = 1.0 / sqrt(1.0 - beta2);
-  const double bp = v3_dot(pb, lv_vec(o));
-  const double gamma2 = beta2 > 1e-14 ? (gamma - 1.0) / beta2 : 0.0;
-  const double s = gamma2 * bp + gamma * o.t;
-  return {gamma * (o.t + bp), o.x + s * pb.x, o.y + s * pb.y, o.z + s * pb.z};
-}
 __device__ __forceinline__ double kin_inv_mass(LV p) {
   return sqrt(fabs(p.t * p.t - (p.x * p.x + p.y * p.y + p.z * p.z)));
+}
+
+// The same algebra with what several daughters, decays and topologies share
+// formed once, and with products by 1 / sqrt instead of square roots and
+// divisions.
+//
+// A particle at rest frame: p / m^2-free form of rest_vector.  For p = (E, p)
+// of mass m, o boosted into its rest frame is
+//   t' = (E t - p.o) / m,   o' = o - p (t + t') / (E + m).
+struct KBoost {
+  double t, x, y, z, im, g;  // momentum, 1 / m, 1 / (E + m)
+};
+__device__ __forceinline__ KBoost kin_frame(LV p) {
+  const double m2 = p.t * p.t - (p.x * p.x + p.y * p.y + p.z * p.z);
+  const double im = prsqrt(m2);
+  return {p.t, p.x, p.y, p.z, im, 1.0 / (p.t + m2 * im)};
+}
+__device__ __forceinline__ LV kin_to_rest(const KBoost& f, LV o) {
+  const double t = (f.t * o.t - (f.x * o.x + f.y * o.y + f.z * o.z)) * f.im;
+  const double s = (o.t + t) * f.g;
+  return {t, o.x - s * f.x, o.y - s * f.y, o.z - s * f.z};
+}
+// Orthonormal axes of a decay (z along the mother's momentum, x as
+// angle_zx_z_getx leaves it) and the length of the momentum z came from
+struct KAxes {
+  V3 x, y, z;
+  double zr;
+};
+// axes of the parent's decay: z along its momentum where it moves
+__device__ __forceinline__ KAxes kin_top_axes(LV p, bool moving_z) {
+  const double p2 = p.x * p.x + p.y * p.y + p.z * p.z;
+  if (!moving_z || sqrt(p2) < 1e-5)
+    return {V3{1.0, 0.0, 0.0}, V3{0.0, 1.0, 0.0}, V3{0.0, 0.0, 1.0}, 1.0};
+  const V3 z = lv_vec(p), y = kin_cross_unit(z, V3{1.0, 0.0, 0.0});
+  return {kin_cross_unit(y, z), y, v3_unit(z), sqrt(p2)};
+}
+struct KAngles {
+  double alpha, beta;
+  KAxes axes;
+};
+// momenta (anti)parallel to the axis: the reference's fallback axes (out of
+// line, by value: the common path's values stay in registers)
+PWA_NOINLINE __device__ KAngles kin_angles_degenerate(KAxes a, V3 v) {
+  const V3 z1 = {a.z.x * a.zr, a.z.y * a.zr, a.z.z * a.zr};
+  KAngles r;
+  kin_angle_zx_z_getx(z1, a.x, v, &r.alpha, &r.beta, &r.axes.x);
+  r.axes.z = v3_unit(v);
+  r.axes.y = v3_cross(r.axes.z, r.axes.x);
+  r.axes.zr = sqrt(v3_dot(v, v));
+  return r;
+}
+// Euler angles (alpha, beta) of momentum v in axes a, and v's own axes:
+// with (vx, vy, vz) its components, alpha = atan2(vy, vx), beta =
+// atan2(sqrt(vx^2 + vy^2), vz), y' = unit(z x v), x' = y' x z'
+__device__ __forceinline__ KAngles kin_angles(const KAxes& a, V3 v) {
+  const double vx = v3_dot(v, a.x), vy = v3_dot(v, a.y), vz = v3_dot(v, a.z);
+  const double pt2 = vx * vx + vy * vy;
+  if (pt2 * (a.zr * a.zr) < 1e-28) return kin_angles_degenerate(a, v);
+  const double it = prsqrt(pt2), ca = vx * it, sa = vy * it;
+  const double p2 = pt2 + vz * vz, ip = prsqrt(p2);
+  KAngles r;
+  r.alpha = atan2(vy, vx);
+  r.beta = atan2(pt2 * it, vz);
+  r.axes.z = {v.x * ip, v.y * ip, v.z * ip};
+  r.axes.y = {ca * a.y.x - sa * a.x.x, ca * a.y.y - sa * a.x.y, ca * a.y.z - sa * a.x.z};
+  r.axes.x = v3_cross(r.axes.y, r.axes.z);
+  r.axes.zr = p2 * ip;
+  return r;
+}
+// alpha in [-pi, pi] folded into [-pi, pi) (first daughter) or [-2 pi, 0)
+__device__ __forceinline__ double kin_fold_first(double a) {
+  return a >= 3.141592653589793 ? a - 6.283185307179586 : a;
+}
+__device__ __forceinline__ double kin_fold_second(double a) {
+  return a >= 0.0 ? a - 6.283185307179586 : a;
 }
 
 __device__ __forceinline__ double2 c2mul(double2 a, double2 b) {

@@ -2655,23 +2655,48 @@ extern "C" __global__ void pwa_reduce_multi(const double* __restrict__ tile_part
 // Dataset step on the device (model_kin / model_genbod are generated per
 // model).  One event per thread, grid-stride, FP64.
 //
-// pwa_fields_from_p4: final-state momenta, rows (4 f + c) of P4 with stride
-// ld_in (c = E, px, py, pz; finals in dat_order; parent rest frame) -> every
-// plan field, row j of OUT with stride ld_out (plan order).
-extern "C" __global__ void __launch_bounds__(PWA_TPB)
-    pwa_fields_from_p4(const double* __restrict__ P4, long long n, long long ld_in,
-                       double* __restrict__ out, long long ld_out) {
+// pwa_fields_from_p4: final-state momenta -> every plan field, row j of OUT
+// with stride ld_out (plan order).  Component c (E, px, py, pz) of final f
+// (dat_order) of event i is P4[i se + f sf + c sc], so rows (4 f + c) of a
+// component-major array and an (N, n_final, 4) tensor of any strides are read
+// as they are, without a transposed copy; pairs = 1: components adjacent and
+// 16-byte aligned (two 16-byte loads a final).  Bound: FP64 arithmetic and
+// its latency (two atan2 and two reciprocal square roots per decay).
+// 1e6 four-body events, whole call: 192 us; 1.41 ms with the copy, the axes
+// of every daughter of every topology normalised step by step and all fields
+// held to the end in 255 registers.
+struct FieldRows {  // field j of one event straight to its row
+  double* p;
+  long long ld;
+  __device__ __forceinline__ double& operator[](int j) const { return p[j * ld]; }
+};
+// three blocks per SM: four-body 203 us against 248 at two and 204 at four
+// (D -> K pi pi 103, 129 and 92)
+#ifndef PWA_KIN_MINB
+#define PWA_KIN_MINB 3
+#endif
+extern "C" __global__ void __launch_bounds__(PWA_TPB, PWA_KIN_MINB)
+    pwa_fields_from_p4(const double* __restrict__ P4, long long n, long long se, long long sf,
+                       long long sc, int pairs, double* __restrict__ out, long long ld_out) {
   for (long long i = (long long)blockIdx.x * PWA_TPB + threadIdx.x; i < n;
        i += (long long)gridDim.x * PWA_TPB) {
     LV P[PWA_NFIN];
+    const double* p = P4 + i * se;
+    if (pairs) {
 #pragma unroll
-    for (int f = 0; f < PWA_NFIN; ++f)
-      P[f] = LV{__ldg(P4 + (4LL * f) * ld_in + i), __ldg(P4 + (4LL * f + 1) * ld_in + i),
-                __ldg(P4 + (4LL * f + 2) * ld_in + i), __ldg(P4 + (4LL * f + 3) * ld_in + i)};
-    double F[PWA_NFIELD];
+      for (int f = 0; f < PWA_NFIN; ++f) {
+        const double2 a = __ldg(reinterpret_cast<const double2*>(p + f * sf));
+        const double2 b = __ldg(reinterpret_cast<const double2*>(p + f * sf) + 1);
+        P[f] = LV{a.x, a.y, b.x, b.y};
+      }
+    } else {
+#pragma unroll
+      for (int f = 0; f < PWA_NFIN; ++f)
+        P[f] = LV{__ldg(p + f * sf), __ldg(p + f * sf + sc), __ldg(p + f * sf + 2 * sc),
+                  __ldg(p + f * sf + 3 * sc)};
+    }
+    FieldRows F{out + i, ld_out};
     model_kin(P, F);
-#pragma unroll
-    for (int j = 0; j < PWA_NFIELD; ++j) out[(long long)j * ld_out + i] = F[j];
   }
 }
 
@@ -2730,10 +2755,8 @@ extern "C" __global__ void __launch_bounds__(PWA_TPB)
     event_uniforms(seed, (unsigned long long)__ldg(idx + i), U);
     LV P[PWA_NFIN];
     model_genbod(U, P);
-    double F[PWA_NFIELD];
+    FieldRows F{out + i, ld_out};
     model_kin(P, F);
-#pragma unroll
-    for (int j = 0; j < PWA_NFIELD; ++j) out[(long long)j * ld_out + i] = F[j];
     if (P4) {
 #pragma unroll
       for (int f = 0; f < PWA_NFIN; ++f) {

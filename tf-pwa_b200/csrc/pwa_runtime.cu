@@ -813,17 +813,30 @@ int pwa_eval_pdf(pwa_plan* h, const double* consts, int precision, long long beg
   return PWA_OK;
 }
 
-int pwa_fields_from_p4(pwa_plan* h, const double* p4, long long n, long long ld_in, double* out,
-                       long long ld_out, void* stream) {
+int pwa_fields_from_strided(pwa_plan* h, const double* p4, long long n, long long stride_event,
+                            long long stride_final, long long stride_comp, double* out,
+                            long long ld_out, void* stream) {
   if (!h) return PWA_ERR_ARG;
-  if (n < 0 || (n > 0 && (!p4 || !out || ld_in < n || ld_out < n)))
+  if (n < 0 || (n > 0 && (!p4 || !out || ld_out < n)) || stride_event < 0 || stride_final < 0 ||
+      stride_comp < 0)
     return set_err(h, PWA_ERR_ARG, "invalid fields_from_p4 arguments");
   if (n == 0) return PWA_OK;
   cudaStream_t s = (cudaStream_t)stream;
-  void* args[] = {(void*)&p4, &n, &ld_in, &out, &ld_out};
+  int pairs = stride_comp == 1 && stride_event % 2 == 0 && stride_final % 2 == 0 &&
+              (size_t)p4 % 16 == 0;
+  void* args[] = {(void*)&p4, &n, &stride_event, &stride_final, &stride_comp, &pairs, &out,
+                  &ld_out};
   long long nb = (n + h->tpb - 1) / h->tpb;
   if (nb > 16LL * h->sms) nb = 16LL * h->sms;
   return launch(h, h->k.fields_from_p4, dim3((int)nb), dim3(h->tpb), args, s);
+}
+
+int pwa_fields_from_p4(pwa_plan* h, const double* p4, long long n, long long ld_in, double* out,
+                       long long ld_out, void* stream) {
+  if (!h) return PWA_ERR_ARG;
+  if (n > 0 && ld_in < n) return set_err(h, PWA_ERR_ARG, "invalid fields_from_p4 arguments");
+  return pwa_fields_from_strided(h, p4, n, 1, 4 * (ld_in > 0 ? ld_in : 0), ld_in > 0 ? ld_in : 0,
+                                 out, ld_out, stream);
 }
 
 int pwa_toy_select(pwa_plan* h, const double* consts, unsigned long long seed, long long first,

@@ -88,6 +88,7 @@ def load_library(path=LIB_PATH):
     lib.pwa_eval_noalloc.argtypes = [vp, dp, vp, vp, vp, ll, ll, ll, vp, vp]
     ull = ctypes.c_ulonglong
     lib.pwa_fields_from_p4.argtypes = [vp, vp, ll, ll, vp, ll, vp]
+    lib.pwa_fields_from_strided.argtypes = [vp, vp, ll, ll, ll, ll, vp, ll, vp]
     lib.pwa_toy_select.argtypes = [vp, dp, ull, ll, ll, ctypes.c_double, i, vp, vp]
     lib.pwa_toy_fields.argtypes = [vp, ull, vp, ll, vp, ll, vp, ll, vp]
     lib.pwa_hessian_cached.argtypes = [vp, dp, ctypes.c_double, ctypes.c_double, vp, dp, dp, dp]
@@ -138,7 +139,8 @@ EXPORTED = ("pwa_plan_create", "pwa_plan_destroy", "pwa_compile_only", "pwa_prec
             "pwa_eval_cached_enqueue", "pwa_set_param_layout", "pwa_pieces_cached",
             "pwa_nll_grad_cached", "pwa_set_cached_variant", "pwa_pool_reserve",
             "pwa_pool_alloc", "pwa_pool_free", "pwa_pool_fill", "pwa_pieces_multi",
-            "pwa_eval_noalloc", "pwa_fields_from_p4", "pwa_toy_select", "pwa_toy_fields",
+            "pwa_eval_noalloc", "pwa_fields_from_p4", "pwa_fields_from_strided",
+            "pwa_toy_select", "pwa_toy_fields",
             "pwa_hessian_cached", "pwa_hessian_cached_exact", "pwa_hess_sums_cached",
             "pwa_shape_cache", "pwa_eval_shapecache", "pwa_eval_shapecache_enqueue",
             "pwa_read_dat", "pwa_hostprog_create", "pwa_hostprog_destroy",
@@ -1363,11 +1365,13 @@ class Engine:
             if self.plan.cp_trans:
                 sgn = torch.where(ch > 0, 1.0, -1.0).to(torch.float64)[:, None, None]
                 p4 = torch.cat([p4[:, :, :1], p4[:, :, 1:] * sgn], 2)
-        soa = p4.permute(1, 2, 0).reshape(-1, n).contiguous()
+        if p4.dim() != 3 or p4.shape[1] < self.code.kin.nfin or p4.shape[2] < 4:
+            raise ValueError(f"momenta of shape {tuple(p4.shape)}: (N, {self.code.kin.nfin}, 4) "
+                             "expected")
         out = torch.empty((self.plan.n_fields, n), dtype=torch.float64, device=p4.device)
-        self._check(load_library().pwa_fields_from_p4(self.h, soa.data_ptr(), n, n,
-                                                      out.data_ptr(), n, 0),
-                    "pwa_fields_from_p4")
+        self._check(load_library().pwa_fields_from_strided(self.h, p4.data_ptr(), n, *p4.stride(),
+                                                           out.data_ptr(), n, 0),
+                    "pwa_fields_from_strided")
         if ch is not None and ci is not None:
             out[ci] = ch
         return out

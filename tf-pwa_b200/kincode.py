@@ -64,123 +64,156 @@ class KinCode:
         # per level of k bodies: k - 2 sorted uniforms + (cos theta, phi) per
         # splitting; then the phase-space and amplitude accept draws
         self.ndraw = sum(3 * len(b) - 4 for _, b in self.levels) + 2
-        self.needs_su2 = any("/aligned/" in f for f in plan.fields)
 
     # ------------------------------------------------------------ kinematics
+    def _wanted(self, sk):
+        """What the fields of pass ``sk`` read: helicity angles as
+        {(topology, decay, particle): [(field, "alpha" | "beta")]}, masses as
+        {node name: field}, and the finals whose SU(2) path is needed as
+        {(topology, final)} (alignment fields and their reference)."""
+        plan = self.plan
+        angles, masses, su2 = {}, {}, set()
+        for fi, full_name in enumerate(plan.fields):
+            if fi == plan.charge_index:
+                continue
+            k, fname = split_swap(full_name)
+            parts = fname.split("/")
+            if k != sk:
+                continue
+            if parts[0] == "m":
+                masses[parts[1]] = fi
+                continue
+            t = int(parts[0])
+            topo = plan.topos[t]
+            dec = next(d for d in topo.chain if topo.decay_name(d) == parts[1])
+            part = next(o for o in dec.outs if topo.node[o] == parts[2])
+            if parts[3] == "aligned":
+                su2.add((t, part))
+                ref = plan.align_ref[str(part)]
+                su2.add((ref, next(o for o in plan.topos[ref].chain.outs
+                                   if str(o) == str(part))))
+            else:
+                angles.setdefault((t, dec, part), []).append((fi, parts[3]))
+        return angles, masses, su2
+
+    def _emit_pass(self, e, pexpr, sk):
+        """Masses and helicity angles of one set of momenta (``pexpr``:
+        final -> LV expression), each field written as soon as it is formed;
+        what several topologies share (the parent's frame, finals in it) is
+        emitted once.  Returns per topology the names of the finals' SU(2)
+        rotation and boost products."""
+        plan = self.plan
+        want, masses, su2 = self._wanted(sk)
+        n = [0]
+
+        def tmp(prefix):
+            n[0] += 1
+            return f"p{sk}{prefix}{n[0]}"
+
+        def lsum(parts):
+            expr = parts[0]
+            for p in parts[1:]:
+                expr = f"lv_add({expr}, {p})"
+            return expr
+
+        for topo in plan.topos:
+            for p in topo.chain.inner:
+                fi = masses.pop(topo.node[p], None)
+                if fi is not None:
+                    fs = [pexpr[str(f)] for f in topo.chain.final_set(p)]
+                    e(f"  F[{fi}] = kin_inv_mass({lsum(fs)});")
+        outs = [str(o) for o in plan.topos[0].chain.outs]
+        top, frame, axes = tmp("top"), tmp("fr"), tmp("ax")
+        e(f"  const LV {top} = {lsum([pexpr[o] for o in outs])};")
+        e(f"  const KBoost {frame} = kin_frame({top});")
+        e(f"  const KAxes {axes} = kin_top_axes({top}, {'true' if plan.random_z else 'false'});")
+        in_top = {}
+        for o in outs:
+            in_top[o] = tmp("q")
+            e(f"  const LV {in_top[o]} = kin_to_rest({frame}, {pexpr[o]});")
+        result = []
+        for t, topo in enumerate(plan.topos):
+            chain = topo.chain
+            decay_of = {d.core: d for d in chain}
+            path = {}  # particles on the way to a final whose SU(2) product is needed
+            for tt, o in su2:
+                if tt == t:
+                    p = o
+                    while p != chain.top:
+                        path[p] = True
+                        p = next(d for d in chain if p in d.outs).core
+            rmat, bmat = {}, {}
+
+            def need(d):
+                """Whether the momenta of decay d's daughters are read."""
+                return any((t, d, j) in want or j in path or (j in decay_of and need(decay_of[j]))
+                           for j in d.outs)
+
+            def walk(d, vec, ax, bm, rm):
+                """Decay d with the finals' momenta ``vec`` in its mother's
+                rest frame, the mother's axes and SU(2) products."""
+                for i, j in enumerate(d.outs):
+                    inner = j in decay_of and need(decay_of[j])
+                    if not ((t, d, j) in want or j in path or inner):
+                        continue
+                    if j in decay_of:
+                        v = tmp("n")
+                        e(f"  const LV {v} = {lsum([vec[str(f)] for f in chain.final_set(j)])};")
+                    else:
+                        v = vec[str(j)]
+                    a, x = tmp("a"), tmp("x")
+                    e(f"  const KAngles {x} = kin_angles({ax}, lv_vec({v}));")
+                    e(f"  const double {a} = kin_fold_{'first' if i == 0 else 'second'}"
+                      f"({x}.alpha);")
+                    b, x = f"{x}.beta", f"{x}.axes"
+                    for fi, kind in want.get((t, d, j), ()):
+                        e(f"  F[{fi}] = {a if kind == 'alpha' else b};")
+                    nb = nr = None
+                    if j in path:
+                        nb, nr = tmp("B"), tmp("R")
+                        e(f"  const SU2 {nb} = su2_boost_z_from_p({v});")
+                        e(f"  const SU2 {nr} = " + (
+                            f"su2_mul(su2_rot_yz({b}, {a}), su2_mul({bm}, {rm}));" if bm
+                            else f"su2_rot_yz({b}, {a});"))
+                        rmat[j], bmat[j] = nr, nb
+                    if inner:
+                        fr = tmp("fr")
+                        e(f"  const KBoost {fr} = kin_frame({v});")
+                        dj = decay_of[j]
+                        sub = {}
+                        for q in dj.outs:
+                            if not ((t, dj, q) in want or q in path
+                                    or (q in decay_of and need(decay_of[q]))):
+                                continue
+                            for f in (chain.final_set(q) if q in decay_of else [q]):
+                                sub[str(f)] = tmp("r")
+                                e(f"  const LV {sub[str(f)]} = kin_to_rest({fr}, {vec[str(f)]});")
+                        walk(dj, sub, x, nb, nr)
+
+            walk(decay_of[chain.top], in_top, axes, None, None)
+            result.append((rmat, bmat))
+        return result
+
     def _emit_kin(self, e):
         plan = self.plan
         fin = {o: i for i, o in enumerate(self.order)}
+        # unswapped momenta, then one relabelling per swap (final pi takes the
+        # momentum of src[pi], three-momentum reversed in the CP-conjugate ones)
+        all_frames = [self._emit_pass(e, {o: f"P[{fin[o]}]" for o in fin}, 0)]
+        for k, sw in enumerate(plan.swaps):
+            pe = {}
+            for o in fin:
+                q = f"P[{fin[sw['src'].get(o, o)]}]"
+                pe[o] = f"LV{{{q}.t, -{q}.x, -{q}.y, -{q}.z}}" if sw["neg"] else q
+            all_frames.append(self._emit_pass(e, pe, k + 1))
         cnt = [0]
+        aligned = {}  # Euler angle names of the alignment rotations emitted so far
 
         def tmp(prefix):
             cnt[0] += 1
             return f"{prefix}{cnt[0]}"
 
-        def build_frames(pexpr):
-            """Frames of every topology from the finals' momenta pexpr."""
-            frames = []
-            for t, topo in enumerate(plan.topos):
-                chain = topo.chain
-                mom = {}
-                for o in chain.outs:
-                    mom[o] = pexpr[str(o)]
-
-                def lsum(parts):
-                    expr = parts[0]
-                    for p in parts[1:]:
-                        expr = f"lv_add({expr}, {p})"
-                    return expr
-
-                for p in chain.inner:
-                    v = tmp(f"t{t}_n")
-                    e(f"  const LV {v} = {lsum([mom[f] for f in chain.final_set(p)])};")
-                    mom[p] = v
-                v = tmp(f"t{t}_top")
-                e(f"  const LV {v} = {lsum([mom[f] for f in chain.outs])};")
-                mom[chain.top] = v
-                top = chain.top
-                # successive rest-frame momenta (same visiting order as the host code)
-                part, core_map = {}, {}
-                decays = list(chain)
-                remaining = set(chain.inner) | set(chain.outs)
-                while decays:
-                    later = []
-                    for d in decays:
-                        if d.core == top:
-                            pr, src = mom[top], mom
-                        elif d.core in core_map:
-                            par = part[core_map[d.core]]
-                            pr, src = par[d.core], par
-                        else:
-                            later.append(d)
-                            continue
-                        rp = {}
-                        for j in d.outs:
-                            core_map[j] = d
-                            v = tmp(f"t{t}_r")
-                            e(f"  const LV {v} = kin_rest_vector({pr}, {src[j]});")
-                            rp[j] = v
-                            remaining.discard(j)
-                        for j in sorted(remaining, key=str):
-                            if j in src:
-                                v = tmp(f"t{t}_r")
-                                e(f"  const LV {v} = kin_rest_vector({pr}, {src[j]});")
-                                rp[j] = v
-                        part[d] = rp
-                    decays = later
-                # helicity angles, frames, SU(2) bookkeeping
-                set_x = {top: "V3{1.0, 0.0, 0.0}"}
-                set_z = {top: "V3{0.0, 0.0, 1.0}"}
-                if plan.random_z:
-                    # a moving parent's flight direction is the z axis
-                    # (tf_pwa/cal_angle.py:431-438)
-                    bz = tmp(f"t{t}_bz")
-                    e(f"  V3 {bz} = lv_vec({mom[top]});")
-                    e(f"  if (sqrt(v3_dot({bz}, {bz})) < 1e-5) {bz} = V3{{0.0, 0.0, 1.0}};")
-                    set_z[top] = bz
-                angles, rmat, bmat = {}, {}, {}
-                decays = list(chain)
-                while decays:
-                    later = []
-                    for d in decays:
-                        if d.core not in set_x:
-                            later.append(d)
-                            continue
-                        bias = -math.pi
-                        for j in d.outs:
-                            z2 = tmp(f"t{t}_z")
-                            a, b, x2 = tmp(f"t{t}_a"), tmp(f"t{t}_b"), tmp(f"t{t}_x")
-                            e(f"  const V3 {z2} = lv_vec({part[d][j]});")
-                            e(f"  double {a}, {b}; V3 {x2};")
-                            e(f"  kin_angle_zx_z_getx({set_z[d.core]}, {set_x[d.core]}, {z2}, "
-                              f"&{a}, &{b}, &{x2});")
-                            e(f"  {a} = kin_fold({a}, {_f(bias)});")
-                            bias -= math.pi
-                            set_x[j], set_z[j] = x2, z2
-                            angles[(d, j)] = (a, b)
-                            if self.needs_su2:
-                                bm, rm = tmp(f"t{t}_B"), tmp(f"t{t}_R")
-                                e(f"  const SU2 {bm} = su2_boost_z_from_p({part[d][j]});")
-                                if d.core in rmat:
-                                    e(f"  const SU2 {rm} = su2_mul(su2_rot_yz({b}, {a}), "
-                                      f"su2_mul({bmat[d.core]}, {rmat[d.core]}));")
-                                else:
-                                    e(f"  const SU2 {rm} = su2_rot_yz({b}, {a});")
-                                bmat[j], rmat[j] = bm, rm
-                    decays = later
-                frames.append((topo, angles, rmat, bmat, mom))
-            return frames
-
-        # unswapped momenta, then one relabelling per swap (final pi takes the
-        # momentum of src[pi], three-momentum reversed in the CP-conjugate ones)
-        all_frames = [build_frames({o: f"P[{fin[o]}]" for o in fin})]
-        for sw in plan.swaps:
-            pe = {}
-            for o in fin:
-                q = f"P[{fin[sw['src'].get(o, o)]}]"
-                pe[o] = f"LV{{{q}.t, -{q}.x, -{q}.y, -{q}.z}}" if sw["neg"] else q
-            all_frames.append(build_frames(pe))
-        # the plan's fields
+        # alignment angles, and the charge
         for fi, full_name in enumerate(plan.fields):
             if fi == plan.charge_index:
                 # the event's charge is data, not kinematics: +1 here (the
@@ -188,32 +221,26 @@ class KinCode:
                 e(f"  F[{fi}] = 1.0;")
                 continue
             sk, fname = split_swap(full_name)
-            frames = all_frames[sk]
             parts = fname.split("/")
-            if parts[0] == "m":
-                for topo, angles, rmat, bmat, mom in frames:
-                    hit = [p for p in topo.chain.inner if topo.node[p] == parts[1]]
-                    if hit:
-                        e(f"  F[{fi}] = kin_inv_mass({mom[hit[0]]});")
-                        break
-                continue
+            if parts[-2] != "aligned":
+                continue  # written with its decay
             tidx = int(parts[0])
-            topo, angles, rmat, bmat, mom = frames[tidx]
+            topo = plan.topos[tidx]
             dec = [d for d in topo.chain if topo.decay_name(d) == parts[1]][0]
             part = [o for o in dec.outs if topo.node[o] == parts[2]][0]
-            if parts[3] == "aligned":
-                ref_t = plan.align_ref[str(part)]
-                rtopo, _, rr, rb, _ = frames[ref_t]
-                rpart = [o for o in rtopo.chain.outs if str(o) == str(part)][0]
+            rmat, bmat = all_frames[sk][tidx]
+            ref_t = plan.align_ref[str(part)]
+            rr, rb = all_frames[sk][ref_t]
+            rpart = [o for o in plan.topos[ref_t].chain.outs if str(o) == str(part)][0]
+            if (sk, tidx, part) not in aligned:
                 m, al, be, ga = tmp("al_M"), tmp("al_a"), tmp("al_b"), tmp("al_g")
                 e(f"  const SU2 {m} = su2_mul(su2_mul({rb[rpart]}, su2_mul({rr[rpart]}, "
                   f"su2_inv({rmat[part]}))), su2_inv({bmat[part]}));")
                 e(f"  double {al}, {be}, {ga};")
                 e(f"  su2_euler({m}, &{al}, &{be}, &{ga});")
-                e(f"  F[{fi}] = {dict(alpha=al, beta=be, gamma=ga)[parts[4]]};")
-            else:
-                a, b = angles[(dec, part)]
-                e(f"  F[{fi}] = {a if parts[3] == 'alpha' else b};")
+                aligned[(sk, tidx, part)] = (al, be, ga)
+            al, be, ga = aligned[(sk, tidx, part)]
+            e(f"  F[{fi}] = {dict(alpha=al, beta=be, gamma=ga)[parts[4]]};")
 
     # ------------------------------------------------------------ GENBOD
     def _build_levels(self):
@@ -346,8 +373,9 @@ class KinCode:
              f"#define PWA_NDRAW {self.ndraw}", f"#define PWA_HAS_GENBOD {int(self.ok)}"]
         body = []
         self._emit_kin(body.append)
-        L.append("__device__ __forceinline__ void model_kin(const LV (&P)[PWA_NFIN], "
-                 "double (&F)[PWA_NFIELD]) {")
+        # F: an array of the fields, or a sink whose [] gives where one goes
+        L.append("template <class Fields>\n__device__ __forceinline__ void model_kin("
+                 "const LV (&P)[PWA_NFIN], Fields& F) {")
         L += body
         L.append("}\n")
         L.append("__device__ __forceinline__ double model_genbod(const double (&U)[PWA_NDRAW], "
