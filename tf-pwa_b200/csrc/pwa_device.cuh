@@ -229,6 +229,30 @@ __device__ __forceinline__ void warp_reduce_scatter(float (&v)[P], int lane) {
   warp_rs_step<P, 16, P>(v, lane);
 }
 
+// The warp sums of C values per lane (C a power of two, at most 16), summed
+// over lane bits in the order 16, 8, 4, 2, 1 as above (bitwise the same sums
+// for any C): halving while more than one value is live, then butterflies.
+// Lane l returns the sum of entry l / (32 / C).  C - 1 + log2(32 / C)
+// shuffles.
+template <int C, int O>
+__device__ __forceinline__ float warp_sum_entries(const float (&v)[C], int lane) {
+  if constexpr (C == 1) {
+    float s = v[0];
+#pragma unroll
+    for (int o = O; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
+  } else {
+    const bool up = (lane & O) != 0;
+    float h[C / 2];
+#pragma unroll
+    for (int j = 0; j < C / 2; ++j) {
+      const float keep = up ? v[j + C / 2] : v[j], send = up ? v[j] : v[j + C / 2];
+      h[j] = keep + __shfl_xor_sync(0xffffffffu, send, O);
+    }
+    return warp_sum_entries<C / 2, O / 2>(h, lane);
+  }
+}
+
 // clip_log and its derivative in FP64
 __device__ __forceinline__ double clip_log(double x, double* dx) {
   const double eps = 1e-6;

@@ -1521,16 +1521,20 @@ extern "C" __global__ void __launch_bounds__(PWA_TPB, 4)
 // PWA_GPAD / 32 FP64 accumulators across tiles instead of 2 * PWA_NCOL:
 // the register footprint no longer grows with the number of columns.
 #define PWA_GPAD ((2 * PWA_NCOL + 31) / 32 * 32)
-// With 2 * PWA_NCOL <= 16 the sensitivities form one group of 16 values:
-// four halving steps leave lanes 2i and 2i + 1 with halves of entry i, one
-// more shuffle gives both the warp sum (16 shuffles instead of 31).
-// Otherwise PWA_GPAD / 32 groups of 32: lane l holds entry 32 m + l of group m.
+// With 2 * PWA_NCOL <= 16 the sensitivities form one group of PWA_RSN values
+// (2 * PWA_NCOL rounded up to a power of two): entry i ends on the
+// 32 / PWA_RSN lanes from (32 / PWA_RSN) i (16 shuffles for 16 values, 6 for
+// four, instead of 31).  Otherwise PWA_GPAD / 32 groups of 32: lane l holds
+// entry 32 m + l of group m.
 #define PWA_RS16 (2 * PWA_NCOL <= 16)
+#define PWA_RSN (2 * PWA_NCOL <= 2 ? 2 : 2 * PWA_NCOL <= 4 ? 4 : 2 * PWA_NCOL <= 8 ? 8 : 16)
 #define PWA_MG (PWA_RS16 ? 1 : PWA_GPAD / 32)
 __device__ __forceinline__ int rs_entry(int m, int lane) {
-  return PWA_RS16 ? (lane >> 1) : 32 * m + lane;
+  return PWA_RS16 ? lane / (32 / PWA_RSN) : 32 * m + lane;
 }
-__device__ __forceinline__ bool rs_owner(int lane) { return PWA_RS16 ? !(lane & 1) : true; }
+__device__ __forceinline__ bool rs_owner(int lane) {
+  return PWA_RS16 ? lane % (32 / PWA_RSN) == 0 : true;
+}
 
 struct CoupParam {  // couplings from the kernel's parameter block
   const CCoup& c;
@@ -1541,7 +1545,7 @@ struct CoupShared {  // couplings staged in shared memory (read per event, not h
   __device__ __forceinline__ double operator()(int i) const { return c[i]; }
 };
 struct CoupGlobal {  // couplings from global memory (one row per request)
-  const double* __restrict__ c;
+  const double* c;
   __device__ __forceinline__ double operator()(int i) const { return __ldg(c + i); }
 };
 
@@ -1639,17 +1643,16 @@ __device__ __forceinline__ double cached_event_rs(const float2 (&v)[PWA_NF], dou
   }
 #if PWA_RS16
   {
-    float g[16];
+    float g[PWA_RSN];
 #pragma unroll
-    for (int q = 0; q < 16; ++q) g[q] = 0.f;
+    for (int q = 0; q < PWA_RSN; ++q) g[q] = 0.f;
 #pragma unroll
     for (int j = 0; j < PWA_NF; ++j) {
       const int k = pwa_fk[j], o = pwa_fo[j];
       g[2 * k] = fmaf(br[o], v[j].x, fmaf(-bi[o], v[j].y, g[2 * k]));
       g[2 * k + 1] = fmaf(br[o], v[j].y, fmaf(bi[o], v[j].x, g[2 * k + 1]));
     }
-    warp_rs_step<16, 16, 16>(g, lane);
-    gs[0] = g[0] + __shfl_xor_sync(0xffffffffu, g[0], 1);
+    gs[0] = warp_sum_entries<PWA_RSN, 16>(g, lane);
   }
 #else
 #pragma unroll
@@ -2235,19 +2238,18 @@ extern "C" __global__ void __launch_bounds__(PWA_PTS_WARPS * 32, 1)
       const double s0 = warp_sum((double)(w * cl));
       if (lane == 0) my[m * NA] += s0;
 #if PWA_RS16
-      float g[16];
+      float g[PWA_RSN];
 #pragma unroll
-      for (int q = 0; q < 16; ++q) g[q] = 0.f;
+      for (int q = 0; q < PWA_RSN; ++q) g[q] = 0.f;
 #pragma unroll
       for (int j = 0; j < PWA_NF; ++j) {
         const int k = pwa_fk[j], o = pwa_fo[j];
         g[2 * k] = fmaf(br[o], v[j].x, fmaf(-bi[o], v[j].y, g[2 * k]));
         g[2 * k + 1] = fmaf(br[o], v[j].y, fmaf(bi[o], v[j].x, g[2 * k + 1]));
       }
-      warp_rs_step<16, 16, 16>(g, lane);
-      const float gs = g[0] + __shfl_xor_sync(0xffffffffu, g[0], 1);
-      const int idx = lane >> 1;
-      if (!(lane & 1) && idx < NG) my[m * NA + 1 + idx] += (double)gs;
+      const float gs = warp_sum_entries<PWA_RSN, 16>(g, lane);
+      const int idx = rs_entry(0, lane);
+      if (rs_owner(lane) && idx < NG) my[m * NA + 1 + idx] += (double)gs;
 #else
 #pragma unroll
       for (int mg = 0; mg < PWA_GPAD / 32; ++mg) {
@@ -2470,12 +2472,11 @@ extern "C" __global__ void __launch_bounds__(PWA_TPB, PWA_HESS_MINB)
       {
         const float f1 = (float)(w * d1);
 #if PWA_RS16
-        float gq[16];
+        float gq[PWA_RSN];
 #pragma unroll
-        for (int q = 0; q < 16; ++q)
+        for (int q = 0; q < PWA_RSN; ++q)
           gq[q] = q < W ? ((q & 1) ? -f1 * row[K + (q >> 1)] : f1 * row[q >> 1]) : 0.f;
-        warp_rs_step<16, 16, 16>(gq, lane);
-        acc_s1[0] += (double)(gq[0] + __shfl_xor_sync(0xffffffffu, gq[0], 1));
+        acc_s1[0] += (double)warp_sum_entries<PWA_RSN, 16>(gq, lane);
 #else
 #pragma unroll
         for (int m = 0; m < PWA_GPAD / 32; ++m) {
@@ -2588,66 +2589,176 @@ extern "C" __global__ void __launch_bounds__(PWA_TPB, PWA_HESS_MINB)
 
 // ---------------------------------------------------------------------------
 // Many fits in one launch (serving).  Each fit's data-event column cache is a
-// run of tiles in a shared pool (same tile layout as above).  The launch gets
-// a work list of (request, pool tile) pairs covering the tiles of every fit
-// with a pending evaluation; each block evaluates work tiles with that
-// request's couplings and writes one row of per-tile sums.  pwa_reduce_multi
-// then sums each request's rows in the fit's own tile order, so a fit's
-// result does not depend on which other fits share the launch.  Per-tile
-// column sums use the warp reduce-scatter of pwa_eval_cached_wred.
-extern "C" __global__ void __launch_bounds__(PWA_TPB, PWA_WRED_MINB)
-    pwa_eval_multi(const double* __restrict__ ck, const int* __restrict__ work_req,
-                   const long long* __restrict__ work_tile, long long n_work,
-                   const float2* __restrict__ Fc, const double* __restrict__ Wc,
-                   double* __restrict__ tile_part) {
+// run of tiles in a shared pool (same tile layout as above).  A pending
+// evaluation (request) is cut into chunks of csize[r] consecutive tiles, a
+// number that depends on the fit's own tile count alone.  A block takes a
+// run of chunks with about 1 / gridDim of all tiles; a warp keeps its sums in
+// registers over a chunk and writes them as one row, without a barrier.
+// Then the block counts its chunks in; the warp that completes a group of
+// PWA_MGROUP chunks of a fit sums the group's rows, the one that completes
+// the fit's groups sums those into out (mapped host memory), the last fit
+// writes the call number: one launch, no work list and no copy back, and a
+// fit's sums depend neither on the other fits nor on the grid.  Column sums
+// per warp and tile as in pwa_eval_cached_wred.
+//
+// meta (8-byte words): chunk_beg, tile_beg, group_beg [n_req + 1 each] (sums
+// over the requests before), first_tile[n_req] (in the pool), csize[n_req],
+// then the couplings, 2 * PWA_NCOL doubles per request.  rows: NA sums per
+// (chunk, warp), then per group.  count: group counters, request counters,
+// finished requests (zero between launches).
+//
+// Bound: at few pairs per event (D -> K pi pi: 24 bytes) by the issue slots
+// and latency of the events' chains (logarithm, division), so eight blocks
+// share an SM (whole rounds of 256 fits, 1.6e7 events: 253 us; 336 at six,
+// 423 at four; loading the next tile ahead costs registers and gains
+// nothing, 282).  With a work list from the host, a row per tile summed in a
+// second launch and the sums copied back, a round took 440 us and takes 226.
+#define PWA_MGROUP 8
+#ifndef PWA_MULTI_MINB
+#define PWA_MULTI_MINB (PWA_NF <= 8 ? 8 : PWA_WRED_MINB)
+#endif
+
+struct MultiMeta {
+  const long long *cbeg, *tbeg, *gbeg, *first, *csize;
+  const double* ck;
+  __device__ __forceinline__ MultiMeta(const long long* m, int n)
+      : cbeg(m), tbeg(cbeg + n + 1), gbeg(tbeg + n + 1), first(gbeg + n + 1), csize(first + n),
+        ck(reinterpret_cast<const double*>(csize + n)) {}
+};
+// the request r and chunk c (over all requests) of the first chunk that
+// starts at or after tile s of all requests' tiles
+__device__ __forceinline__ void multi_first(const MultiMeta& m, int n_req, long long s, int* r,
+                                            long long* c) {
+  int lo = 0;
+  for (int hi = n_req; hi - lo > 1;) {
+    const int mid = (lo + hi) >> 1;
+    if (__ldg(m.tbeg + mid) <= s) lo = mid;
+    else hi = mid;
+  }
+  const long long cs = __ldg(m.csize + lo);
+  *c = __ldg(m.cbeg + lo) + (s - __ldg(m.tbeg + lo) + cs - 1) / cs;
+  *r = *c < __ldg(m.cbeg + lo + 1) ? lo : lo + 1;
+}
+// sums over `n` rows of NA doubles into out[0 .. NA) by one warp: rows
+// strided over the lanes, a fixed shuffle tree
+__device__ __forceinline__ void multi_sum_rows(const double* rows, long long n, double* out,
+                                               int lane) {
   constexpr int NA = PWA_CACHE_NA;
-  constexpr int NG = 2 * PWA_NCOL;
-  __shared__ double red[PWA_TPB / 32][NA];
+#pragma unroll 4
+  for (int j = 0; j < NA; ++j) {
+    double s = 0.0;
+    for (long long r = lane; r < n; r += 32) s += __ldcg(rows + r * NA + j);
+    s = warp_sum(s);
+    if (lane == 0) out[j] = s;
+  }
+}
+
+extern "C" __global__ void __launch_bounds__(PWA_TPB, PWA_MULTI_MINB)
+    pwa_eval_multi(const long long* __restrict__ meta, int n_req, long long n_chunks,
+                   long long n_tiles, long long n_groups, const float2* __restrict__ Fc,
+                   const double* __restrict__ Wc, double* __restrict__ rows,
+                   unsigned int* __restrict__ count, double* __restrict__ out, double seq) {
+  constexpr int NA = PWA_CACHE_NA, NG = 2 * PWA_NCOL, MG = PWA_MG, NW = PWA_TPB / 32;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (long long wi = blockIdx.x; wi < n_work; wi += gridDim.x) {
-    const int r = work_req[wi];
-    const long long t = work_tile[wi];
-    const CoupGlobal cp{ck + (long long)r * 2 * PWA_NCOL};
+  const MultiMeta m(meta, n_req);
+  int r, rb;
+  long long ca, cb;
+  multi_first(m, n_req, n_tiles * blockIdx.x / gridDim.x, &r, &ca);
+  multi_first(m, n_req, n_tiles * (blockIdx.x + 1) / gridDim.x, &rb, &cb);
+  if (ca >= cb) return;
+  const int ra = r;
+  int c = (int)ca, cend = (int)__ldg(m.cbeg + r + 1);
+  long long cs = __ldg(m.csize + r), t = __ldg(m.first + r),
+            te = t + __ldg(m.tbeg + r + 1) - __ldg(m.tbeg + r);
+  t += (ca - __ldg(m.cbeg + r)) * cs;
+  long long t1 = t + cs < te ? t + cs : te;
+  double acc0 = 0.0, accg[MG];
+#pragma unroll
+  for (int q = 0; q < MG; ++q) accg[q] = 0.0;
+#pragma unroll 1
+  while (c < cb) {
     const float2* F = Fc + t * PWA_NF * PWA_TPB + tid;
     float2 v[PWA_NF];
 #pragma unroll
     for (int j = 0; j < PWA_NF; ++j) v[j] = __ldcs(F + j * PWA_TPB);
     const double w = __ldcs(Wc + t * PWA_TPB + tid);
-    float gs[PWA_MG];
-    const double s0 = warp_sum(cached_event_rs(v, w, cp, lane, gs));
-    if (lane == 0) red[warp][0] = s0;
+    const CoupGlobal cp{m.ck + (long long)r * NG};
+    float gs[MG];
+    acc0 += cached_event_rs(v, w, cp, lane, gs);
 #pragma unroll
-    for (int m = 0; m < PWA_MG; ++m) {
-      const int idx = rs_entry(m, lane);
-      if (rs_owner(lane) && idx < NG) red[warp][1 + idx] = (double)gs[m];
-    }
-    __syncthreads();
-    for (int j = tid; j < NA; j += PWA_TPB) {
-      double s = 0.0;
+    for (int q = 0; q < MG; ++q) accg[q] += (double)gs[q];
+    if (++t < t1) continue;
+    // the chunk's row, then the next chunk (and request)
+    double* row = rows + ((long long)c * NW + warp) * NA;
+    acc0 = warp_sum(acc0);
+    if (lane == 0) row[0] = acc0;
+    acc0 = 0.0;
 #pragma unroll
-      for (int w2 = 0; w2 < PWA_TPB / 32; ++w2) s += red[w2][j];
-      tile_part[wi * NA + j] = s;
+    for (int q = 0; q < MG; ++q) {
+      const int idx = rs_entry(q, lane);
+      if (rs_owner(lane) && idx < NG) row[1 + idx] = accg[q];
+      accg[q] = 0.0;
     }
-    __syncthreads();
+    if (++c == cend && c < cb) {
+      ++r;
+      cend = (int)__ldg(m.cbeg + r + 1);
+      cs = __ldg(m.csize + r);
+      t = __ldg(m.first + r);
+      te = t + __ldg(m.tbeg + r + 1) - __ldg(m.tbeg + r);
+    }
+    t1 = t + cs < te ? t + cs : te;
   }
-}
-
-// out[r * NA + j] = sum over rows [row_beg[r], row_beg[r+1]) of tile_part,
-// in row order (one warp per (request, accumulator), lanes strided, fixed
-// shuffle tree).
-extern "C" __global__ void pwa_reduce_multi(const double* __restrict__ tile_part,
-                                            const long long* __restrict__ row_beg, int n_req,
-                                            double* __restrict__ out) {
-  constexpr int NA = PWA_CACHE_NA;
-  const int lane = threadIdx.x & 31;
-  const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
-  for (long long q = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-       q < (long long)n_req * NA; q += warps) {
-    const int r = (int)(q / NA), j = (int)(q % NA);
-    double s = 0.0;
-    for (long long row = row_beg[r] + lane; row < row_beg[r + 1]; row += 32) s += tile_part[row * NA + j];
-    s = warp_sum(s);
-    if (lane == 0) out[q] = s;
+  __threadfence();
+  __syncthreads();
+  // count the block's chunks in: lane l of warp v takes group v + NW l of the
+  // groups that [ca, cb) touches, then 32 NW further
+  double* grow = rows + n_chunks * NW * NA;
+  const long long ga = __ldg(m.gbeg + ra) + (ca - __ldg(m.cbeg + ra)) / PWA_MGROUP;
+  const long long gz = __ldg(m.gbeg + r) + (cb - 1 - __ldg(m.cbeg + r)) / PWA_MGROUP;
+  for (long long gw = ga + warp; gw <= gz; gw += 32 * NW) {
+    const long long g = gw + NW * lane;
+    int q = ra;
+    bool full = false;
+    if (g <= gz) {
+      while (__ldg(m.gbeg + q + 1) <= g) ++q;  // the group's request
+      const long long q0 = __ldg(m.cbeg + q), b0 = q0 + (g - __ldg(m.gbeg + q)) * PWA_MGROUP;
+      const long long qe = __ldg(m.cbeg + q + 1);
+      const long long b1 = b0 + PWA_MGROUP < qe ? b0 + PWA_MGROUP : qe;
+      const unsigned mine = (unsigned)((b1 < cb ? b1 : cb) - (b0 > ca ? b0 : ca));
+      full = atomicAdd(count + g, mine) + mine == (unsigned)(b1 - b0);
+    }
+    unsigned todo = __ballot_sync(0xffffffffu, full);
+    while (todo) {
+      const int src = __ffs(todo) - 1;
+      todo &= todo - 1;
+      const long long gg = gw + NW * src;
+      const int qq = __shfl_sync(0xffffffffu, q, src);
+      __threadfence();
+      const long long g0 = __ldg(m.gbeg + qq), ng = __ldg(m.gbeg + qq + 1) - g0;
+      const long long b0 = __ldg(m.cbeg + qq) + (gg - g0) * PWA_MGROUP;
+      const long long qe = __ldg(m.cbeg + qq + 1);
+      const long long b1 = b0 + PWA_MGROUP < qe ? b0 + PWA_MGROUP : qe;
+      multi_sum_rows(rows + b0 * NW * NA, (b1 - b0) * NW, grow + gg * NA, lane);
+      int last = 0;
+      if (lane == 0) {
+        count[gg] = 0u;
+        __threadfence();
+        last = atomicAdd(count + n_groups + qq, 1u) == (unsigned)ng - 1;
+      }
+      if (!__shfl_sync(0xffffffffu, last, 0)) continue;
+      __threadfence();
+      multi_sum_rows(grow + g0 * NA, ng, out + (long long)qq * NA, lane);
+      if (lane == 0) {
+        count[n_groups + qq] = 0u;
+        __threadfence_system();  // this fit's sums before its mark
+        if (atomicAdd(count + n_groups + n_req, 1u) == (unsigned)n_req - 1) {
+          count[n_groups + n_req] = 0u;
+          __threadfence_system();
+          out[(long long)n_req * NA] = seq;
+        }
+      }
+      __syncwarp();
+    }
   }
 }
 

@@ -40,8 +40,7 @@ struct Kernels {
                eval_cached_direct = nullptr, eval_cached_wred = nullptr, eval_cached_ring2 = nullptr,
                eval_cached_wide = nullptr, eval_cached_tma = nullptr, eval_multi = nullptr,
                gram_colmax = nullptr, gram_tc = nullptr, wait_check = nullptr,
-               fma_f64 = nullptr, fma_f32 = nullptr, eval_points = nullptr, reduce_multi = nullptr,
-               gram_fused = nullptr, eval_cols = nullptr, hess_cached = nullptr, cache_ns_f32 = nullptr, eval_shapecache = nullptr,
+               fma_f64 = nullptr, fma_f32 = nullptr, eval_points = nullptr, gram_fused = nullptr, eval_cols = nullptr, hess_cached = nullptr, cache_ns_f32 = nullptr, eval_shapecache = nullptr,
                fields_from_p4 = nullptr, toy_select = nullptr, toy_fields = nullptr;
 };
 
@@ -87,6 +86,10 @@ struct pwa_plan {
   int cached_variant = -1;
   size_t cached_smem = 0;
   unsigned int* ticket = nullptr;  // [0] finished groups, [1] error flag, [2 + g] group counts
+  // one pinned mapped block: the results below, and pin_batch_cap bytes from
+  // pin_batch for pwa_pieces_multi
+  char *h_pin = nullptr, *d_pin = nullptr;
+  size_t pin_batch = 0, pin_batch_cap = 0;
   double* h_map = nullptr;         // mapped pinned result of the cached kernel
   double* d_map = nullptr;         // its device address
   double* h_map_sc = nullptr;      // mapped result of pwa_eval_shapecache (2 nacc + 2)
@@ -101,14 +104,14 @@ struct pwa_plan {
   long long pool_tiles = 0;
   std::vector<std::pair<long long, long long>> pool_free;  // (first, count), sorted
   std::vector<std::pair<long long, long long>> pool_used;  // (first, count)
-  // batch scratch of pwa_pieces_multi
-  int* d_work_req = nullptr;
-  long long* d_work_tile = nullptr;
-  long long* d_row_beg = nullptr;
-  double* d_ck = nullptr;
-  double* d_tile_part = nullptr;
-  double* d_multi_out = nullptr;
-  long long multi_cap_work = 0, multi_cap_req = 0;
+  // scratch of pwa_pieces_multi: one device block (counters, zero between
+  // launches; arguments; rows) and, for batches beyond pin_batch_cap bytes,
+  // a pinned block of its own (arguments, then the mapped result)
+  char* d_multi = nullptr;
+  long long mcount_cap = 0, mrows_cap = 0;
+  size_t mmeta_cap = 0;
+  char *h_mbig = nullptr, *d_mbig = nullptr;
+  size_t mbig_cap = 0;
   int multi_bps = 0;  // blocks per SM of pwa_eval_multi (0: occupancy limit)
   // multi-point evaluation: device couplings and sums of up to pts_cap points
   double* d_pts = nullptr;
@@ -132,6 +135,15 @@ struct pwa_plan {
   // parameter layout for the C-side chain rule
   int n_vars = 0, n_coup = 0, nfac = 0, n_train = 0;
   std::vector<int> coup_r, coup_i, coup_polar, col_fac, train_idx;
+  // the non-zero d c_k / d (trainable variable) of that layout, variable by
+  // variable: which coupling and part, its power in the column, and the
+  // column's other couplings jac_oth[oth .. oth + n_oth)
+  struct JacEntry {
+    int t, k, coup, comp, power, oth, n_oth;
+  };
+  std::vector<JacEntry> jac;
+  std::vector<int> jac_oth;
+  bool jac_ok = false;  // every trainable variable is a coupling part
   // host program of the evaluations from the variable vector
   // (pwa_set_host_program) and the constant block the floating-shape column
   // cache was built at
@@ -455,7 +467,7 @@ int pwa_plan_create(const char* src, size_t src_len, int n_mass, int n_angle, in
             {"pwa_fields_from_p4", &h->k.fields_from_p4},
             {"pwa_toy_select", &h->k.toy_select},
             {"pwa_toy_fields", &h->k.toy_fields},
-            {"pwa_eval_multi", &h->k.eval_multi},   {"pwa_reduce_multi", &h->k.reduce_multi},
+            {"pwa_eval_multi", &h->k.eval_multi},
             {"pwa_hess_cached", &h->k.hess_cached},
             {"pwa_cache_ns_f32", &h->k.cache_ns_f32},
             {"pwa_eval_shapecache", &h->k.eval_shapecache}};
@@ -469,10 +481,17 @@ int pwa_plan_create(const char* src, size_t src_len, int n_mass, int n_angle, in
   // [0] finished groups, [1] error flag, [2 + g] finished blocks of group g
   CU(cudaMalloc(&h->ticket, kTicketWords * sizeof(unsigned int)));
   CU(cudaMemset(h->ticket, 0, kTicketWords * sizeof(unsigned int)));
-  CU(cudaHostAlloc(&h->h_map, sizeof(double) * (2 * ncol + 4), cudaHostAllocMapped));
-  CU(cudaHostGetDevicePointer((void**)&h->d_map, h->h_map, 0));
-  CU(cudaHostAlloc(&h->h_map_sc, sizeof(double) * (2 * h->nacc + 2), cudaHostAllocMapped));
-  CU(cudaHostGetDevicePointer((void**)&h->d_map_sc, h->h_map_sc, 0));
+  {
+    const size_t b0 = (sizeof(double) * (2 * ncol + 4) + 255) / 256 * 256;
+    h->pin_batch = b0 + (sizeof(double) * (2 * h->nacc + 2) + 255) / 256 * 256;
+    h->pin_batch_cap = 256 * 1024;
+    CU(cudaHostAlloc(&h->h_pin, h->pin_batch + h->pin_batch_cap, cudaHostAllocMapped));
+    CU(cudaHostGetDevicePointer((void**)&h->d_pin, h->h_pin, 0));
+    h->h_map = (double*)h->h_pin;
+    h->d_map = (double*)h->d_pin;
+    h->h_map_sc = (double*)(h->h_pin + b0);
+    h->d_map_sc = (double*)(h->d_pin + b0);
+  }
   // no call number yet: pinned memory may come back from a closed plan with
   // that plan's last number in it
   h->h_map[2 * ncol + 2] = -1.0;
@@ -489,17 +508,12 @@ int pwa_plan_destroy(pwa_plan* h) {
   if (h->ticket) cudaFree(h->ticket);
   if (h->pool_f) cudaFree(h->pool_f);
   if (h->pool_w) cudaFree(h->pool_w);
-  if (h->d_work_req) cudaFree(h->d_work_req);
-  if (h->d_work_tile) cudaFree(h->d_work_tile);
-  if (h->d_row_beg) cudaFree(h->d_row_beg);
-  if (h->d_ck) cudaFree(h->d_ck);
-  if (h->d_tile_part) cudaFree(h->d_tile_part);
-  if (h->d_multi_out) cudaFree(h->d_multi_out);
+  if (h->d_multi) cudaFree(h->d_multi);
+  if (h->h_mbig) cudaFreeHost(h->h_mbig);
   if (h->d_pts) cudaFree(h->d_pts);
   if (h->d_hsum) cudaFree(h->d_hsum);
   if (h->scache) cudaFree(h->scache);
-  if (h->h_map) cudaFreeHost(h->h_map);
-  if (h->h_map_sc) cudaFreeHost(h->h_map_sc);
+  if (h->h_pin) cudaFreeHost(h->h_pin);
   if (h->lib) cudaLibraryUnload(h->lib);
   delete h;
   return PWA_OK;
@@ -1480,6 +1494,32 @@ int pwa_set_param_layout(pwa_plan* h, int n_vars, int n_coup, const int* coup_r,
   h->coup_polar.assign(coup_polar, coup_polar + n_coup);
   h->col_fac.assign(col_fac, col_fac + h->ncol * nfac);
   h->train_idx.assign(train_idx, train_idx + n_train);
+  h->jac.clear();
+  h->jac_oth.clear();
+  h->jac_ok = true;
+  for (int t = 0; t < n_train; ++t) {
+    int j = -1, comp = 0;
+    for (int q = 0; q < n_coup && j < 0; ++q) {
+      if (coup_r[q] == train_idx[t]) j = q, comp = 0;
+      else if (coup_i[q] == train_idx[t]) j = q, comp = 1;
+    }
+    if (j < 0) {
+      h->jac_ok = false;
+      continue;
+    }
+    for (int k = 0; k < h->ncol; ++k) {
+      pwa_plan::JacEntry e{t, k, j, comp, 0, (int)h->jac_oth.size(), 0};
+      for (int f = 0; f < nfac; ++f) {
+        const int q = col_fac[k * nfac + f];
+        if (q < 0) continue;
+        if (q == j && e.power++ == 0) continue;  // one factor is differentiated
+        h->jac_oth.push_back(q);
+      }
+      e.n_oth = (int)h->jac_oth.size() - e.oth;
+      if (e.power) h->jac.push_back(e);
+      else h->jac_oth.resize(e.oth);
+    }
+  }
   return PWA_OK;
 }
 
@@ -1491,32 +1531,45 @@ inline cplx cmulh(cplx a, cplx b) { return {a.r * b.r - a.i * b.i, a.r * b.i + a
 }  // namespace
 
 namespace {
-// Column couplings of one parameter vector (layout of pwa_set_param_layout).
-void column_couplings(const pwa_plan* h, const double* vars, std::vector<cplx>* z,
-                      double* ck) {
-  z->resize(h->n_coup);
+// Couplings z, their d z / d r (ph) and the column couplings ck of one
+// parameter vector (layout of pwa_set_param_layout).  prev: a parameter
+// vector whose z, ph are at zp, php; couplings with the same two values are
+// taken from there (the fits of a batch differ in few of them).
+void column_couplings(const pwa_plan* h, const double* vars, cplx* z, cplx* ph, double* ck,
+                      const double* prev = nullptr, const cplx* zp = nullptr,
+                      const cplx* php = nullptr) {
   for (int j = 0; j < h->n_coup; ++j) {
-    const double r = vars[h->coup_r[j]], p = vars[h->coup_i[j]];
-    (*z)[j] = h->coup_polar[j] ? cplx{r * std::cos(p), r * std::sin(p)} : cplx{r, p};
+    const int vr = h->coup_r[j], vi = h->coup_i[j];
+    const double r = vars[vr], p = vars[vi];
+    if (prev && prev[vr] == r && prev[vi] == p) {
+      z[j] = zp[j];
+      ph[j] = php[j];
+      continue;
+    }
+    ph[j] = h->coup_polar[j] ? cplx{std::cos(p), std::sin(p)} : cplx{1.0, 0.0};
+    z[j] = h->coup_polar[j] ? cplx{r * ph[j].r, r * ph[j].i} : cplx{r, p};
   }
   for (int k = 0; k < h->ncol; ++k) {
     cplx c{1.0, 0.0};
     for (int f = 0; f < h->nfac; ++f) {
       const int j = h->col_fac[k * h->nfac + f];
-      if (j >= 0) c = cmulh(c, (*z)[j]);
+      if (j >= 0) c = cmulh(c, z[j]);
     }
     ck[2 * k] = c.r;
     ck[2 * k + 1] = c.i;
   }
 }
 
-// Piece vector from the data sums sd[1 + 2*ncol] of one parameter vector:
-// MC term from the Gram matrix and the chain rule to the trainable variables.
-int pieces_from_sums(pwa_plan* h, const double* vars, const std::vector<cplx>& z,
-                     const double* ck, const double* sd, double sw, double mc_share,
-                     double* out) {
+// What of the piece vector of one parameter vector needs no data sums: the
+// Jacobian entries J (h->jac), the MC integral from the Gram matrix and its
+// derivatives.  Runs while the device forms the data sums.
+int pieces_before(pwa_plan* h, const cplx* z, const cplx* ph, const double* ck, double sw,
+                  double mc_share, cplx* J, double* out) {
+  if (!h->jac_ok)
+    return set_err(h, PWA_ERR_ARG, "trainable variable is not a coupling (cached mode)");
   const int K = h->ncol, P = h->n_train;
-  std::vector<cplx> Gm(K, cplx{0, 0});
+  thread_local std::vector<cplx> Gm;
+  Gm.assign(K, cplx{0, 0});
   double I = 0.0;
   for (int k = 0; k < K; ++k) {
     cplx acc{0, 0};
@@ -1530,48 +1583,44 @@ int pieces_from_sums(pwa_plan* h, const double* vars, const std::vector<cplx>& z
     Gm[k] = acc;
     I += acc.r * ck[2 * k] - acc.i * ck[2 * k + 1];
   }
-  out[0] = sd[0];
   out[1] = I * mc_share;
   out[2] = sw;
-  for (int t = 0; t < P; ++t) {
-    const int v = h->train_idx[t];
-    int j = -1, comp = 0;
-    for (int q = 0; q < h->n_coup && j < 0; ++q) {
-      if (h->coup_r[q] == v) j = q, comp = 0;
-      else if (h->coup_i[q] == v) j = q, comp = 1;
-    }
-    if (j < 0) return set_err(h, PWA_ERR_ARG, "trainable variable is not a coupling (cached mode)");
-    const double r = vars[h->coup_r[j]], p = vars[h->coup_i[j]];
-    cplx dz;
-    if (h->coup_polar[j])
-      dz = comp == 0 ? cplx{std::cos(p), std::sin(p)} : cplx{-r * std::sin(p), r * std::cos(p)};
-    else
-      dz = comp == 0 ? cplx{1, 0} : cplx{0, 1};
-    double gd = 0.0, gm = 0.0;
-    for (int k = 0; k < K; ++k) {
-      int cnt = 0;
-      cplx others{1.0, 0.0};
-      for (int f = 0; f < h->nfac; ++f) {
-        const int q = h->col_fac[k * h->nfac + f];
-        if (q < 0) continue;
-        if (q == j && cnt == 0) {
-          ++cnt;
-          continue;
-        }
-        if (q == j) ++cnt;
-        others = cmulh(others, z[q]);
-      }
-      if (!cnt) continue;
-      cplx J = cmulh(others, dz);
-      J.r *= cnt;
-      J.i *= cnt;
-      const cplx Gd{sd[1 + 2 * k], sd[2 + 2 * k]};
-      gd += 2.0 * (J.r * Gd.r - J.i * Gd.i);
-      gm += 2.0 * (J.r * Gm[k].r - J.i * Gm[k].i);
-    }
-    out[3 + t] = gd;
-    out[3 + P + t] = gm * mc_share;
+  for (int t = 0; t < P; ++t) out[3 + P + t] = 0.0;
+  for (size_t n = 0; n < h->jac.size(); ++n) {
+    const pwa_plan::JacEntry& e = h->jac[n];
+    cplx others{1.0, 0.0};
+    for (int f = 0; f < e.n_oth; ++f) others = cmulh(others, z[h->jac_oth[e.oth + f]]);
+    const cplx dz = e.comp == 0 ? ph[e.coup]
+                    : h->coup_polar[e.coup] ? cplx{-z[e.coup].i, z[e.coup].r}
+                                            : cplx{0, 1};
+    J[n] = cmulh(others, dz);
+    J[n].r *= e.power;
+    J[n].i *= e.power;
+    out[3 + P + e.t] += 2.0 * (J[n].r * Gm[e.k].r - J[n].i * Gm[e.k].i);
   }
+  for (int t = 0; t < P; ++t) out[3 + P + t] *= mc_share;
+  return PWA_OK;
+}
+
+// The rest, from the data sums sd[1 + 2*ncol].
+void pieces_after(const pwa_plan* h, const cplx* J, const double* sd, double* out) {
+  const int P = h->n_train;
+  out[0] = sd[0];
+  for (int t = 0; t < P; ++t) out[3 + t] = 0.0;
+  for (size_t n = 0; n < h->jac.size(); ++n) {
+    const pwa_plan::JacEntry& e = h->jac[n];
+    out[3 + e.t] += 2.0 * (J[n].r * sd[1 + 2 * e.k] - J[n].i * sd[2 + 2 * e.k]);
+  }
+}
+
+// Piece vector from the data sums sd[1 + 2*ncol] of one parameter vector:
+// MC term from the Gram matrix and the chain rule to the trainable variables.
+int pieces_from_sums(pwa_plan* h, const cplx* z, const cplx* ph, const double* ck,
+                     const double* sd, double sw, double mc_share, double* out) {
+  std::vector<cplx> J(h->jac.size());
+  const int rc = pieces_before(h, z, ph, ck, sw, mc_share, J.data(), out);
+  if (rc) return rc;
+  pieces_after(h, J.data(), sd, out);
   return PWA_OK;
 }
 }  // namespace
@@ -1582,17 +1631,20 @@ int pwa_pieces_cached(pwa_plan* h, const double* vars, double sw, double mc_shar
   if (!vars || !out) return set_err(h, PWA_ERR_ARG, "null argument");
   if (h->n_coup == 0) return set_err(h, PWA_ERR_STATE, "parameter layout not set");
   if (!h->gram_valid) return set_err(h, PWA_ERR_STATE, "MC Gram matrix not built");
-  std::vector<cplx> z;
+  std::vector<cplx> z(h->n_coup), ph(h->n_coup), J(h->jac.size());
   std::vector<double> ck(2 * h->ncol);
-  column_couplings(h, vars, &z, ck.data());
+  column_couplings(h, vars, z.data(), ph.data(), ck.data());
   cudaStream_t s = (cudaStream_t)stream;
   int rc = pwa_eval_cached_enqueue(h, ck.data(), stream);
   if (rc) return rc;
+  const int rc2 = pieces_before(h, z.data(), ph.data(), ck.data(), sw, mc_share, J.data(), out);
   wait_cached(h, s);
   const double* sd = nullptr;
   rc = cached_result(h, &sd);
   if (rc) return rc;
-  return pieces_from_sums(h, vars, z, ck.data(), sd, sw, mc_share, out);
+  if (rc2) return rc2;
+  pieces_after(h, J.data(), sd, out);
+  return PWA_OK;
 }
 
 // ------------------------------------------------------------------ pool
@@ -1689,86 +1741,121 @@ int pwa_pieces_multi(pwa_plan* h, int n_req, const long long* first_tile, const 
   if (h->n_coup == 0) return set_err(h, PWA_ERR_STATE, "parameter layout not set");
   if (!h->gram_valid) return set_err(h, PWA_ERR_STATE, "MC Gram matrix not built");
   const int K = h->ncol, NA = 1 + 2 * K, P = h->n_train;
-  long long n_work = 0;
-  std::vector<long long> row_beg(n_req + 1, 0);
+  cudaStream_t s = (cudaStream_t)stream;
+  // chunks of a fit's tiles, from its own tile count: about 128 chunks, at
+  // most 16 tiles each (a lone fit of 1e6 events still has 489 to spread over
+  // the device, a round of hundreds of fits keeps rows few)
+  constexpr int kGroup = 8;  // PWA_MGROUP
+  const int NW = h->tpb / 32;
+  auto chunk_tiles = [](long long nt) {
+    const long long c = (nt + 127) / 128;
+    return c < 1 ? 1 : c > 16 ? 16LL : c;
+  };
+  const size_t words = 5 * (size_t)n_req + 3 + 2 * (size_t)K * n_req;
+  // pinned arguments and mapped result
+  const size_t meta_bytes = (words * 8 + 255) / 256 * 256;
+  const size_t pin_bytes = meta_bytes + sizeof(double) * ((size_t)n_req * NA + 1);
+  char *h_io = h->h_pin + h->pin_batch, *d_io = h->d_pin + h->pin_batch;
+  if (pin_bytes > h->pin_batch_cap) {
+    if (pin_bytes > h->mbig_cap) {
+      if (h->h_mbig) cudaFreeHost(h->h_mbig);
+      h->h_mbig = h->d_mbig = nullptr;
+      h->mbig_cap = 0;
+      if (cudaHostAlloc(&h->h_mbig, 2 * pin_bytes, cudaHostAllocMapped) != cudaSuccess)
+        return set_err(h, PWA_ERR_OOM, "allocation of the batch arguments failed");
+      CU(cudaHostGetDevicePointer((void**)&h->d_mbig, h->h_mbig, 0));
+      h->mbig_cap = 2 * pin_bytes;
+    }
+    h_io = h->h_mbig;
+    d_io = h->d_mbig;
+  }
+  long long* cbeg = (long long*)h_io;
+  long long *tbeg = cbeg + n_req + 1, *gbeg = tbeg + n_req + 1, *first = gbeg + n_req + 1,
+            *cs = first + n_req;
+  double* ck = (double*)(cs + n_req);
+  long long n_chunks = 0, n_work = 0, n_groups = 0;
   for (int r = 0; r < n_req; ++r) {
     if (first_tile[r] < 0 || n_tiles[r] <= 0 || first_tile[r] + n_tiles[r] > h->pool_tiles)
       return set_err(h, PWA_ERR_ARG, "request tile run outside the pool");
-    row_beg[r] = n_work;
+    cbeg[r] = n_chunks;
+    tbeg[r] = n_work;
+    gbeg[r] = n_groups;
+    first[r] = first_tile[r];
+    cs[r] = chunk_tiles(n_tiles[r]);
+    const long long nc = (n_tiles[r] + cs[r] - 1) / cs[r];
     n_work += n_tiles[r];
+    n_chunks += nc;
+    n_groups += (nc + kGroup - 1) / kGroup;
   }
-  row_beg[n_req] = n_work;
+  cbeg[n_req] = n_chunks;
+  tbeg[n_req] = n_work;
+  gbeg[n_req] = n_groups;
+  const long long n_rows = (n_chunks * NW + n_groups) * NA;
   // grow scratch (serving set-up; steady state allocates nothing)
-  if (n_work > h->multi_cap_work || n_req > h->multi_cap_req) {
-    const long long cw = n_work > h->multi_cap_work ? 2 * n_work : h->multi_cap_work;
-    const long long cr = n_req > h->multi_cap_req ? 2LL * n_req : h->multi_cap_req;
-    cudaFree(h->d_work_req);
-    cudaFree(h->d_work_tile);
-    cudaFree(h->d_row_beg);
-    cudaFree(h->d_ck);
-    cudaFree(h->d_tile_part);
-    cudaFree(h->d_multi_out);
-    h->d_work_req = nullptr;
-    h->d_work_tile = nullptr;
-    h->d_row_beg = nullptr;
-    h->d_ck = nullptr;
-    h->d_tile_part = nullptr;
-    h->d_multi_out = nullptr;
-    h->multi_cap_work = h->multi_cap_req = 0;
-    if (cudaMalloc(&h->d_work_req, sizeof(int) * cw) != cudaSuccess ||
-        cudaMalloc(&h->d_work_tile, sizeof(long long) * cw) != cudaSuccess ||
-        cudaMalloc(&h->d_row_beg, sizeof(long long) * (cr + 1)) != cudaSuccess ||
-        cudaMalloc(&h->d_ck, sizeof(double) * 2 * K * cr) != cudaSuccess ||
-        cudaMalloc(&h->d_tile_part, sizeof(double) * NA * cw) != cudaSuccess ||
-        cudaMalloc(&h->d_multi_out, sizeof(double) * NA * cr) != cudaSuccess)
+  const long long n_count = n_groups + n_req + 1;
+  if (n_rows > h->mrows_cap || n_count > h->mcount_cap || words * 8 > h->mmeta_cap) {
+    if (h->d_multi) cudaFree(h->d_multi);
+    h->d_multi = nullptr;
+    h->mrows_cap = h->mcount_cap = 0;
+    h->mmeta_cap = 0;
+    const long long cc = (2 * n_count + 63) / 64 * 64, cr = 2 * n_rows;
+    const size_t cm = 2 * meta_bytes;
+    if (cudaMalloc(&h->d_multi, sizeof(unsigned int) * cc + cm + sizeof(double) * cr) !=
+        cudaSuccess)
       return set_err(h, PWA_ERR_OOM, "cudaMalloc of the batch scratch failed");
-    h->multi_cap_work = cw;
-    h->multi_cap_req = cr;
+    CU(cudaMemsetAsync(h->d_multi, 0, sizeof(unsigned int) * cc, s));
+    h->mcount_cap = cc;
+    h->mmeta_cap = cm;
+    h->mrows_cap = cr;
   }
-  std::vector<int> wreq(n_work);
-  std::vector<long long> wtile(n_work);
-  std::vector<double> ck(2 * K * (size_t)n_req);
-  std::vector<std::vector<cplx>> zs(n_req);
+  unsigned int* d_count = (unsigned int*)h->d_multi;
+  char* d_meta = h->d_multi + sizeof(unsigned int) * h->mcount_cap;
+  double* d_rows = (double*)(d_meta + h->mmeta_cap);
+  double *h_res = (double*)(h_io + meta_bytes), *d_res = (double*)(d_io + meta_bytes);
+  const size_t nc = h->n_coup;
+  std::vector<cplx> zs(nc * n_req), phs(nc * n_req);
   for (int r = 0; r < n_req; ++r) {
-    for (long long q = 0; q < n_tiles[r]; ++q) {
-      wreq[row_beg[r] + q] = r;
-      wtile[row_beg[r] + q] = first_tile[r] + q;
-    }
-    column_couplings(h, vars + (size_t)r * h->n_vars, &zs[r], ck.data() + 2 * K * (size_t)r);
+    const double* v = vars + (size_t)r * h->n_vars;
+    column_couplings(h, v, &zs[nc * r], &phs[nc * r], ck + 2 * K * (size_t)r,
+                     r ? v - h->n_vars : nullptr, r ? &zs[nc * (r - 1)] : nullptr,
+                     r ? &phs[nc * (r - 1)] : nullptr);
   }
-  cudaStream_t s = (cudaStream_t)stream;
-  CU(cudaMemcpyAsync(h->d_work_req, wreq.data(), sizeof(int) * n_work, cudaMemcpyHostToDevice, s));
-  CU(cudaMemcpyAsync(h->d_work_tile, wtile.data(), sizeof(long long) * n_work,
-                     cudaMemcpyHostToDevice, s));
-  CU(cudaMemcpyAsync(h->d_row_beg, row_beg.data(), sizeof(long long) * (n_req + 1),
-                     cudaMemcpyHostToDevice, s));
-  CU(cudaMemcpyAsync(h->d_ck, ck.data(), sizeof(double) * ck.size(), cudaMemcpyHostToDevice, s));
+  CU(cudaMemcpyAsync(d_meta, h_io, words * 8, cudaMemcpyHostToDevice, s));
   int per_sm = 0;
   CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)h->k.eval_multi, h->tpb, 0));
   if (per_sm < 1) per_sm = 1;
   if (h->multi_bps > 0 && h->multi_bps < per_sm) per_sm = h->multi_bps;
   long long nb = (long long)per_sm * h->sms;
-  if (nb > n_work) nb = n_work;
-  void* a1[] = {&h->d_ck, &h->d_work_req, &h->d_work_tile, &n_work, &h->pool_f, &h->pool_w,
-                &h->d_tile_part};
+  if (nb > n_chunks) nb = n_chunks;
+  h->seq += 1.0;
+  double seq = h->seq;
+  const volatile double* mark = h_res + (size_t)n_req * NA;
+  h_res[(size_t)n_req * NA] = -1.0;  // the mark's place follows the request count
+  void* a1[] = {&d_meta, &n_req, &n_chunks, &n_work, &n_groups, &h->pool_f, &h->pool_w,
+                &d_rows, &d_count, &d_res, &seq};
   int rc = launch(h, h->k.eval_multi, dim3((int)nb), dim3(h->tpb), a1, s);
   if (rc) return rc;
-  long long nq = (long long)n_req * NA;
-  int rb = (int)((nq + 7) / 8);
-  if (rb > 8 * h->sms) rb = 8 * h->sms;
-  void* a2[] = {&h->d_tile_part, &h->d_row_beg, &n_req, &h->d_multi_out};
-  rc = launch(h, h->k.reduce_multi, dim3(rb), dim3(256), a2, s);
-  if (rc) return rc;
-  std::vector<double> sums((size_t)NA * n_req);
-  CU(cudaMemcpyAsync(sums.data(), h->d_multi_out, sizeof(double) * sums.size(),
-                     cudaMemcpyDeviceToHost, s));
-  CU(cudaStreamSynchronize(s));
-  for (int r = 0; r < n_req; ++r) {
-    rc = pieces_from_sums(h, vars + (size_t)r * h->n_vars, zs[r], ck.data() + 2 * K * (size_t)r,
-                          sums.data() + (size_t)NA * r, sw[r], mc_share,
-                          out + (size_t)r * (3 + 2 * P));
-    if (rc) return rc;
+  // the Gram part and the Jacobians while the device forms the data sums
+  std::vector<cplx> J(h->jac.size() * (size_t)n_req);
+  for (int r = 0; r < n_req && !rc; ++r)
+    rc = pieces_before(h, &zs[nc * r], &phs[nc * r], ck + 2 * K * (size_t)r, sw[r], mc_share,
+                       J.data() + h->jac.size() * r, out + (size_t)r * (3 + 2 * P));
+  const auto w0 = std::chrono::steady_clock::now();
+  for (unsigned it = 1; *mark != seq; ++it)
+    if ((it & 4095u) == 0 &&
+        std::chrono::duration<double>(std::chrono::steady_clock::now() - w0).count() > 1.0) {
+      CU(cudaStreamSynchronize(s));
+      break;
+    }
+  std::atomic_thread_fence(std::memory_order_acquire);
+  if (*mark != seq) {
+    cudaMemset(d_count, 0, sizeof(unsigned int) * h->mcount_cap);
+    return set_err(h, PWA_ERR_CUDA, "batch evaluation did not complete (stale result)");
   }
+  if (rc) return rc;
+  for (int r = 0; r < n_req; ++r)
+    pieces_after(h, J.data() + h->jac.size() * r, h_res + (size_t)r * NA,
+                 out + (size_t)r * (3 + 2 * P));
   return PWA_OK;
 }
 
@@ -1830,10 +1917,12 @@ int pwa_pieces_points(pwa_plan* h, int n_pts, const double* vars, double sw, dou
   cudaStream_t s = (cudaStream_t)stream;
   const int K = h->ncol, NA = 1 + 2 * K, P = h->n_train;
   const int per = points_per_launch(h);
-  std::vector<std::vector<cplx>> zs(n_pts);
+  const size_t nc = h->n_coup;
+  std::vector<cplx> zs(nc * n_pts), phs(nc * n_pts);
   std::vector<double> ck((size_t)n_pts * 2 * K), sums((size_t)n_pts * NA);
   for (int m = 0; m < n_pts; ++m)
-    column_couplings(h, vars + (size_t)m * h->n_vars, &zs[m], ck.data() + (size_t)m * 2 * K);
+    column_couplings(h, vars + (size_t)m * h->n_vars, &zs[nc * m], &phs[nc * m],
+                     ck.data() + (size_t)m * 2 * K);
   for (int m0 = 0; m0 < n_pts; m0 += per) {
     const int cnt = n_pts - m0 < per ? n_pts - m0 : per;
     const int rc = eval_points_chunk(h, ck.data() + (size_t)m0 * 2 * K, cnt, s,
@@ -1841,7 +1930,7 @@ int pwa_pieces_points(pwa_plan* h, int n_pts, const double* vars, double sw, dou
     if (rc) return rc;
   }
   for (int m = 0; m < n_pts; ++m) {
-    const int rc = pieces_from_sums(h, vars + (size_t)m * h->n_vars, zs[m],
+    const int rc = pieces_from_sums(h, &zs[nc * m], &phs[nc * m],
                                     ck.data() + (size_t)m * 2 * K, sums.data() + (size_t)m * NA,
                                     sw, mc_share, out + (size_t)m * (3 + 2 * P));
     if (rc) return rc;
@@ -2063,9 +2152,9 @@ int pwa_hess_sums_cached(pwa_plan* h, const double* vars, void* stream, double* 
   if (!vars || !out) return set_err(h, PWA_ERR_ARG, "null argument");
   if (h->fcache_n <= 0) return set_err(h, PWA_ERR_STATE, "no column cache (call pwa_cache_data)");
   if (h->n_coup == 0) return set_err(h, PWA_ERR_STATE, "parameter layout not set");
-  std::vector<cplx> z;
+  std::vector<cplx> z(h->n_coup), ph(h->n_coup);
   std::vector<double> ck(2 * h->ncol);
-  column_couplings(h, vars, &z, ck.data());
+  column_couplings(h, vars, z.data(), ph.data(), ck.data());
   return hess_sums(h, ck.data(), (cudaStream_t)stream, out);
 }
 
@@ -2078,9 +2167,9 @@ int pwa_hessian_cached_exact(pwa_plan* h, const double* vars, double sw, void* s
   if (h->fcache_n <= 0) return set_err(h, PWA_ERR_STATE, "no column cache (call pwa_cache_data)");
   if (h->n_coup == 0) return set_err(h, PWA_ERR_STATE, "parameter layout not set");
   if (!h->gram_valid) return set_err(h, PWA_ERR_STATE, "MC Gram matrix not built");
-  std::vector<cplx> z;
+  std::vector<cplx> z(h->n_coup), ph(h->n_coup);
   std::vector<double> ck(2 * h->ncol), hs((size_t)hess_na(h));
-  column_couplings(h, vars, &z, ck.data());
+  column_couplings(h, vars, z.data(), ph.data(), ck.data());
   int rc = hess_sums(h, ck.data(), (cudaStream_t)stream, hs.data());
   if (rc) return rc;
   return hessian_from_hsums(h, vars, z, ck.data(), hs.data(), sw, out_nll, out_grad, out_hess);
