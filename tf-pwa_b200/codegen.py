@@ -630,6 +630,83 @@ class ModelCode:
         else:
             e(f"  const cpx<R> BW_c{ci} = cmk<R>(R(1), R(0));")
 
+    def _emit_shape_values(self, e):
+        """Body of ``model_bw`` (FP64).  A running-width Breit-Wigner takes
+        one square root and one division: with p = (m^2 - s^2)(m^2 - d^2),
+        s, d = mb +- mc, and u = (2 m)^2, q^2 = p / u, so
+        q^2L / B_L(q^2) = p^L / P with P the homogeneous polynomial
+        sum c_k p^k u^(L-k), and m0 Gamma(m) = Y / w with Y = 2 K sqrt(p) p^L,
+        w = u P (no q0: Y = K u^L, w = m P); then with a = (m0^2 - m^2) w and
+        D = a^2 + Y^2 the value is (a + i Y) w / D, and 1 / w and w / D both
+        follow from 1 / (D w)."""
+        seen = {}
+        for ci, c in enumerate(self.group):
+            cf = self._cf(ci)
+
+            def dmass(p):
+                return f"xm{cf['mass'][p]}" if p in c.inner else repr(float(p.mass))
+
+            other = [p for p in c.inner if p.lineshape_kind() in ("BW", "BWR2")]
+            prod = []
+            if other:
+                e(f"  cpx<R> BW_{ci};")
+                e("  {")
+                self._emit_lineshapes(e, ci)
+                e(f"  BW_{ci} = BW_c{ci};")
+                for si, p in enumerate(self.shape_res):
+                    if p in c.inner and self._first_chain(p) == ci:
+                        tag = f"c{ci}r{c.inner.index(p)}"
+                        e(f"  bw[{si}] = bw_{tag};")
+                        e(f"  e[{si}] = " + (f"cmk<R>(-yi_{tag}, -y_{tag});"
+                                             if p.lineshape_kind() == "BWR2"
+                                             else f"cmk<R>(R(0), y_{tag});"))
+                e("  }")
+                prod.append(f"BW_{ci}")
+            else:
+                for p in c.inner:
+                    if p.lineshape_kind() == "one":
+                        continue
+                    d = c.decay_of(p)
+                    b, cc = d.outs
+                    m = f"xm{cf['mass'][p]}"
+                    key = (p.key(), m, dmass(b), dmass(cc))
+                    if key not in seen:
+                        t = f"s{len(seen)}"
+                        seen[key] = t
+                        L = p.bw_l if p.bw_l is not None else min(d.get_l_list())
+                        co = bprime_coeff(L)
+                        e(f"  const double {t}s = {dmass(b)} + {dmass(cc)}, {t}d = {dmass(b)} - {dmass(cc)};")
+                        e(f"  const double {t}p = {m} > {t}s ? ({m} - {t}s) * ({m} + {t}s) * "
+                          f"({m} - {t}d) * ({m} + {t}d) : 0.0;")
+                        e(f"  const double {t}m2 = {m} * {m}, {t}u = 4.0 * {t}m2;")
+                        poly, up = repr(float(co[0])), ""
+                        for k in range(1, L + 1):
+                            up = f"{t}u" if k == 1 else f"{up} * {t}u"
+                            poly = f"fma({poly}, {t}z, {float(co[k])!r} * ({up}))"
+                        if L:
+                            e(f"  const double {t}z = {t}p * {float(p.d * p.d)!r};")
+                        e(f"  const bool {t}q = C.v[{self._ci(f'{p}.useq')}] != 0.0;")
+                        pl = " * ".join([f"sqrt({t}p)"] + [f"{t}p"] * L)
+                        e(f"  const double {t}Y = C.v[{self._ci(f'{p}.K')}] * ({t}q ? 2.0 * {pl} : "
+                          f"{' * '.join([f'{t}u'] * L) or '1.0'});")
+                        e(f"  const double {t}w = ({t}q ? {t}u : {m}) * ({poly});")
+                        e(f"  const double {t}a = (C.v[{self._ci(f'{p}.m0sq')}] - {t}m2) * {t}w;")
+                        e(f"  const double {t}D = fma({t}a, {t}a, {t}Y * {t}Y);")
+                        e(f"  const double {t}r = 1.0 / ({t}D * {t}w);")
+                        e(f"  const double {t}v = {t}w * {t}w * {t}r;")
+                        e(f"  const cpx<R> {t} = cmk<R>({t}a * {t}v, {t}Y * {t}v);")
+                    t = seen[key]
+                    wn = self._ci(f"{p}.wn") if p.width_norm_applies() else None
+                    prod.append(f"cscale({t}, C.v[{wn}])" if wn else t)
+                    for si, q in enumerate(self.shape_res):
+                        if q == p and self._first_chain(p) == ci:
+                            e(f"  bw[{si}] = {t};")
+                            e(f"  e[{si}] = cmk<R>(R(0), {t}Y * {t}D * {t}r);")
+            v = "cmk<R>(R(1), R(0))"
+            for k, f in enumerate(prod):
+                v = f if k == 0 else f"cmul({v}, {f})"
+            e(f"  BW[{ci}] = {v};")
+
     def _emit_align_forward(self, e, ci, cur, pfx):
         """Contract each aligned final's helicity with D*(aligned angles)."""
         for oi in self._aligned_finals(ci):
@@ -932,20 +1009,44 @@ class ModelCode:
         L.append(ColumnCode(self).source())
         body = []
         self._emit_mass_loads(body.append)
-        for ci in range(len(self.group)):
-            body.append(f"  {{ // chain {ci}")
-            self._emit_lineshapes(body.append, ci)
-            body.append(f"  BW[{ci}] = BW_c{ci};")
-            self._emit_shape_derivs(body.append, ci, "DM[{si}]", "DG[{si}]")
-            body.append("  }")
+        self._emit_shape_values(body.append)
+        L.append("// per event: each chain's lineshape product BW, and per free lineshape its\n"
+                 "// value bw and the factor e with (up to constants of the evaluation)\n"
+                 "//   d bw / d Gamma0 ~ bw e,   d bw / d m0 ~ -2 m0 bw + kappa_m bw e\n"
+                 "template <bool LDG>\n__device__ __forceinline__ void model_bw(\n"
+                 "    const Consts& C, const double* __restrict__ XM, long long ld, long long i,\n"
+                 "    cpx<double>* __restrict__ BW, cpx<double>* __restrict__ bw,\n"
+                 "    cpx<double>* __restrict__ e) {\n  using R = double;")
+        L += body
+        L.append("}\n")
+        # the same with each value times its log-derivatives
         L.append("template <typename R, bool LDG = true>\n__device__ __forceinline__ void model_shapes(\n"
                  "    const Consts& C, const double* __restrict__ XM, long long ld, long long i,\n"
-                 "    cpx<R>* __restrict__ BW, cpx<R>* __restrict__ DM, cpx<R>* __restrict__ DG) {")
-        L += body
+                 "    cpx<R>* __restrict__ BW, cpx<R>* __restrict__ DM, cpx<R>* __restrict__ DG) {\n"
+                 f"  cpx<R> bw[{max(len(self.shape_res), 1)}], e[{max(len(self.shape_res), 1)}];\n"
+                 "  model_bw<LDG>(C, XM, ld, i, BW, bw, e);")
+        for si, p in enumerate(self.shape_res):
+            m0, kap, ig = (f"C.v[{self._ci(f'{p}.{n}')}]" for n in ("m0sq", "kappa_m", "inv_g0"))
+            L.append(f"  {{ const cpx<R> be = cmul(bw[{si}], e[{si}]);\n"
+                     f"    DG[{si}] = cscale(be, {ig});")
+            if p.width_norm_applies():
+                L.append(f"    DG[{si}].re += {ig};")
+            L.append(f"    DM[{si}] = cscale(bw[{si}], -2.0 * sqrt({m0}));\n"
+                     f"    cfma(DM[{si}], {kap}, be); }}")
         L.append("}\n")
         nch, nsr = len(self.group), len(self.shape_res)
         L.append(f"#define PWA_NCHAIN {nch}\n#define PWA_NSRES {nsr}\n"
                  f"#define PWA_SHAPE_CACHE_OK {1 if self.shape_cache_ok else 0}")
+        for nm, key in (("m0sq", "m0sq"), ("kap", "kappa_m"), ("ig", "inv_g0")):
+            L.append(f"__device__ constexpr int pwa_sres_{nm}[PWA_NSRES > 0 ? PWA_NSRES : 1] = {{" +
+                     (", ".join(self._ci(f"{p}.{key}") for p in self.shape_res) or "0") + "};")
+        L.append("__device__ constexpr bool pwa_sres_wn[PWA_NSRES > 0 ? PWA_NSRES : 1] = {" +
+                 (", ".join("true" if p.width_norm_applies() else "false"
+                            for p in self.shape_res) or "false") + "};")
+        has = {(self.columns[k][0], o) for k, o in self._fset}
+        L.append("__device__ constexpr bool pwa_chain_out[PWA_NCHAIN][PWA_NOUT] = {" + ", ".join(
+            "{" + ", ".join("true" if (ci, o) in has else "false" for o in range(self.nout)) + "}"
+            for ci in range(nch)) + "};")
         L.append("__device__ constexpr int pwa_col_chain[PWA_NCOL] = {" +
                  ", ".join(str(ci) for ci, _ in self.columns) + "};")
         rows = [", ".join("1" if p in c.inner else "0" for c in self.group) for p in self.shape_res]

@@ -836,11 +836,15 @@ extern "C" __global__ void __launch_bounds__(PWA_TPB)
 }
 
 struct CRatio {
-  double v[PWA_NCOL];  // r_k: barrier normalisations now / at the cache's setting
+  double v[PWA_NCOL];      // r_k: barrier normalisations now / at the cache's setting
+  double c[2 * PWA_NCOL];  // r_k times the column couplings
 };
 
+// Blocks per SM: the sums of a model set the registers.  Whole evaluations of
+// 2e6 events: D -> K pi pi (9 sums) 57.0 us at 4, 57.7 at 5, 58.8 at 6, 62.9
+// at 8; Lambda_c (23) 155 us at 2, 178 at 3.
 #ifndef PWA_SC_MINB
-#define PWA_SC_MINB 2
+#define PWA_SC_MINB (PWA_NACC <= 12 ? 4 : 2)
 #endif
 // PWA_SC_STAGES 2 (set by the model source where the buffers fit): each warp
 // copies its next 32 events' cached pairs, masses and weights into shared
@@ -882,6 +886,13 @@ __device__ __forceinline__ bool grouped_sum(double* __restrict__ partials,
 __device__ __forceinline__ void publish_result(unsigned int* __restrict__ ticket, int na,
                                                double* __restrict__ out, double seq);
 
+// Bound: FP64 issue and latency (160 FP64 instructions per D -> K pi pi
+// event, one square root and one division per lineshape), then the launch
+// and the reduction's serial tail.  The columns' sums leave out what is
+// constant in an evaluation (r_k, m0, kappa: applied to the sums), a
+// lineshape's two sums come from its chains' amplitudes: 123 -> 106 us for
+// two evaluations of 2e6 events against a form with three divisions and two
+// square roots per lineshape and each column's derivative multiplied out.
 extern "C" __global__ void __launch_bounds__(PWA_TPB, PWA_SC_MINB)
     pwa_eval_shapecache(const Consts C, const CRatio rk, const float2* __restrict__ Fc,
                         const double* __restrict__ XM, const double* __restrict__ W,
@@ -920,92 +931,123 @@ extern "C" __global__ void __launch_bounds__(PWA_TPB, PWA_SC_MINB)
     const long long i = s + lane_s;
     const bool valid = i >= beg && i < end;
     const int col = 32 * warp_s + lane_s;
+    if (!valid) continue;
     // the pairs are read from shared memory where used (both passes), not
     // held in registers
     const float2* vs = reinterpret_cast<const float2*>(cur) + col;
 #define PWA_SC_V(j) vs[(j) * PWA_TPB]
-    cpx<double> BW[PWA_NCHAIN], DM[NS], DG[NS];
-    model_shapes<double, false>(C, cur + PWA_NF * PWA_TPB, PWA_TPB, col, BW, DM, DG);
-    const double w = valid ? cur[(PWA_NF + PWA_SC_NM) * PWA_TPB + col] : 0.0;
+    cpx<double> BW[PWA_NCHAIN], bw[NS], e[NS];
+    model_bw<false>(C, cur + PWA_NF * PWA_TPB, PWA_TPB, col, BW, bw, e);
+    const double w = cur[(PWA_NF + PWA_SC_NM) * PWA_TPB + col];
 #else
   (void)smem_bytes;
   for (long long i = beg + (long long)b * PWA_TPB + threadIdx.x; i < end;
        i += (long long)nb * PWA_TPB) {
-    const long long t = i / PWA_TPB, e = i % PWA_TPB;
-    constexpr bool valid = true;
+    const long long t = i / PWA_TPB, ev = i % PWA_TPB;
     float2 v[PWA_NF];
 #pragma unroll
-    for (int j = 0; j < PWA_NF; ++j) v[j] = __ldcs(Fc + (t * PWA_NF + j) * PWA_TPB + e);
+    for (int j = 0; j < PWA_NF; ++j) v[j] = __ldcs(Fc + (t * PWA_NF + j) * PWA_TPB + ev);
 #define PWA_SC_V(j) v[j]
-    cpx<double> BW[PWA_NCHAIN], DM[NS], DG[NS];
-    model_shapes<double>(C, XM, ld, i, BW, DM, DG);
+    cpx<double> BW[PWA_NCHAIN], bw[NS], e[NS];
+    model_bw<true>(C, XM, ld, i, BW, bw, e);
     const double w = __ldg(W + i);
 #endif
-    // F = s_k Fhat with s_k = r_k BW_ch(k); A_o = sum_k c_k s_k Fhat_k,o
-    double ar[PWA_NOUT], ai[PWA_NOUT];
+    // amplitude of each chain, A_ch,o = BW_ch sum_k (c_k r_k) Fhat_k,o, and
+    // their sum
+    cpx<double> Ac[PWA_NCHAIN][PWA_NOUT];
 #pragma unroll
-    for (int o = 0; o < PWA_NOUT; ++o) ar[o] = ai[o] = 0.0;
+    for (int q = 0; q < PWA_NCHAIN; ++q)
+#pragma unroll
+      for (int o = 0; o < PWA_NOUT; ++o) Ac[q][o] = cmk<double>(0.0, 0.0);
 #pragma unroll
     for (int j = 0; j < PWA_NF; ++j) {
-      const int k = pwa_fk[j], o = pwa_fo[j];
-      const cpx<double> bw = BW[pwa_col_chain[k]];
-      const cpx<double> cs = cmul(cmk<double>(C.v[2 * k], C.v[2 * k + 1]),
-                                  cmk<double>(rk.v[k] * bw.re, rk.v[k] * bw.im));
+      const int k = pwa_fk[j], o = pwa_fo[j], q = pwa_col_chain[k];
       const float2 vj = PWA_SC_V(j);
-      const double x = (double)vj.x, y = (double)vj.y;
-      ar[o] = fma(cs.re, x, fma(-cs.im, y, ar[o]));
-      ai[o] = fma(cs.re, y, fma(cs.im, x, ai[o]));
+      cfmac(Ac[q][o], cmk<double>(rk.c[2 * k], rk.c[2 * k + 1]),
+            cmk<double>((double)vj.x, (double)vj.y));
     }
+    cpx<double> A[PWA_NOUT];
+#pragma unroll
+    for (int o = 0; o < PWA_NOUT; ++o) A[o] = cmk<double>(0.0, 0.0);
+#pragma unroll
+    for (int q = 0; q < PWA_NCHAIN; ++q)
+#pragma unroll
+      for (int o = 0; o < PWA_NOUT; ++o)
+        if (pwa_chain_out[q][o]) {
+          Ac[q][o] = cmul(BW[q], Ac[q][o]);
+          A[o] = cadd(A[o], Ac[q][o]);
+        }
     double f = 0.0;
 #pragma unroll
-    for (int o = 0; o < PWA_NOUT; ++o) f = fma(ar[o], ar[o], fma(ai[o], ai[o], f));
-    double fac;
+    for (int o = 0; o < PWA_NOUT; ++o) f = fma(A[o].re, A[o].re, fma(A[o].im, A[o].im, f));
+    double fac = w;
     if (is_data) {
       double dl;
       const double cl = clip_log(f, &dl);
-      acc[0] = valid ? fma(w, cl, acc[0]) : acc[0];
+      acc[0] = fma(w, cl, acc[0]);
       fac = w * dl;
     } else {
-      acc[0] = valid ? fma(w, f, acc[0]) : acc[0];
-      fac = w;
+      acc[0] = fma(w, f, acc[0]);
     }
-    // g_k = fac s_k sum_o conj(A_o) Fhat_k,o (the pairs j run column by
-    // column);  SR_s = sum over the columns of the chains holding shape s of
-    // c_k g_k
+    // g_k = r_k sum_o (fac conj(A_o) BW_ch) Fhat_k,o, the r_k at the end; a
+    // lineshape's sums need Z = sum_o fac conj(A_o) A_ch,o of its chains
+#pragma unroll
+    for (int o = 0; o < PWA_NOUT; ++o) A[o] = cmk<double>(fac * A[o].re, -fac * A[o].im);
     cpx<double> SR[NS];
 #pragma unroll
     for (int q = 0; q < NS; ++q) SR[q] = cmk<double>(0.0, 0.0);
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-      cpx<double> hk = cmk<double>(0.0, 0.0);
+    for (int q = 0; q < PWA_NCHAIN; ++q) {
+      cpx<double> Z = cmk<double>(0.0, 0.0), B[PWA_NOUT];
+#pragma unroll
+      for (int o = 0; o < PWA_NOUT; ++o)
+        if (pwa_chain_out[q][o]) {
+          cfmac(Z, A[o], Ac[q][o]);
+          B[o] = cmul(A[o], BW[q]);
+        }
 #pragma unroll
       for (int j = 0; j < PWA_NF; ++j) {
-        if (pwa_fk[j] != k) continue;
-        const int o = pwa_fo[j];
+        const int k = pwa_fk[j], o = pwa_fo[j];
+        if (pwa_col_chain[k] != q) continue;
         const float2 vj = PWA_SC_V(j);
         const double x = (double)vj.x, y = (double)vj.y;
-        hk.re = fma(ar[o], x, fma(ai[o], y, hk.re));
-        hk.im = fma(ar[o], y, fma(-ai[o], x, hk.im));
+        acc[1 + 2 * k] = fma(B[o].re, x, fma(-B[o].im, y, acc[1 + 2 * k]));
+        acc[2 + 2 * k] = fma(B[o].re, y, fma(B[o].im, x, acc[2 + 2 * k]));
       }
-      const cpx<double> bw = BW[pwa_col_chain[k]];
-      cpx<double> g = cscale(cmul(cmk<double>(rk.v[k] * bw.re, rk.v[k] * bw.im), hk), fac);
-      g.re = valid ? g.re : 0.0;  // events outside the set (garbage inputs: select, not scale)
-      g.im = valid ? g.im : 0.0;
-      acc[1 + 2 * k] += g.re;
-      acc[2 + 2 * k] += g.im;
-      const cpx<double> cg = cmul(cmk<double>(C.v[2 * k], C.v[2 * k + 1]), g);
 #pragma unroll
-      for (int q = 0; q < PWA_NSRES; ++q)
-        if (pwa_sres_chain[q][pwa_col_chain[k]]) {
-          SR[q].re += cg.re;
-          SR[q].im += cg.im;
-        }
+      for (int s2 = 0; s2 < PWA_NSRES; ++s2)
+        if (pwa_sres_chain[s2][q]) SR[s2] = cadd(SR[s2], Z);
     }
 #pragma unroll
     for (int q = 0; q < PWA_NSRES; ++q) {
-      const double dm = 2.0 * cmul(SR[q], DM[q]).re, dg = 2.0 * cmul(SR[q], DG[q]).re;
-      acc[1 + 2 * K + 2 * q] += valid ? dm : 0.0;
-      acc[2 + 2 * K + 2 * q] += valid ? dg : 0.0;
+      const cpx<double> Wq = cmul(SR[q], bw[q]);
+      const double t2 = Wq.re * e[q].re - Wq.im * e[q].im;
+      if (pwa_sres_wn[q]) {  // the width also scales the value: three sums in two
+        acc[1 + 2 * K + 2 * q] += -2.0 * sqrt(C.v[pwa_sres_m0sq[q]]) * Wq.re +
+                                  C.v[pwa_sres_kap[q]] * t2;
+        acc[2 + 2 * K + 2 * q] += C.v[pwa_sres_ig[q]] * (t2 + SR[q].re);
+      } else {
+        acc[1 + 2 * K + 2 * q] += Wq.re;
+        acc[2 + 2 * K + 2 * q] += t2;
+      }
+    }
+  }
+  // constants of the evaluation, once per thread
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    acc[1 + 2 * k] *= rk.v[k];
+    acc[2 + 2 * k] *= rk.v[k];
+  }
+#pragma unroll
+  for (int q = 0; q < PWA_NSRES; ++q) {
+    const double s1 = acc[1 + 2 * K + 2 * q], s2 = acc[2 + 2 * K + 2 * q];
+    if (pwa_sres_wn[q]) {
+      acc[1 + 2 * K + 2 * q] = 2.0 * s1;
+      acc[2 + 2 * K + 2 * q] = 2.0 * s2;
+    } else {
+      acc[1 + 2 * K + 2 * q] =
+          -4.0 * sqrt(C.v[pwa_sres_m0sq[q]]) * s1 + 2.0 * C.v[pwa_sres_kap[q]] * s2;
+      acc[2 + 2 * K + 2 * q] = 2.0 * C.v[pwa_sres_ig[q]] * s2;
     }
   }
 #if PWA_SC_STAGES > 0

@@ -775,7 +775,12 @@ int pwa_eval_shapecache_enqueue(pwa_plan* h, const double* consts, const double*
   if (h->scache_n != h->n_data + h->n_mc || h->scache_n <= 0)
     return set_err(h, PWA_ERR_STATE, "no floating-shape column cache (call pwa_shape_cache)");
   cudaStream_t s = (cudaStream_t)stream;
+  // ratios, then the column couplings (first constants) times them (CRatio)
   std::vector<double> cbuf = consts_block(h, consts), rbuf(ratio, ratio + h->ncol);
+  for (int k = 0; k < h->ncol; ++k) {
+    rbuf.push_back(consts[2 * k] * ratio[k]);
+    rbuf.push_back(consts[2 * k + 1] * ratio[k]);
+  }
   long long nd = h->n_data, na = h->n_data + h->n_mc, ld = h->ld;
   int bd = h->sc_blocks_data, nb = h->sc_blocks, smem = h->sc_smem;
   h->seq += 1.0;
