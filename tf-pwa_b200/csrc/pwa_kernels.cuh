@@ -34,12 +34,121 @@
 #define PWA_WAIT_LIMIT (1u << 22)
 #endif
 
+// ---------------------------------------------------------------------------
+// Sums over blocks, in a fixed order (results depend only on the inputs and
+// the grid), to mapped host memory, at the end of the kernel that forms them.
+//
+// Blocks per group of the two-level reduction, and the most groups a launch
+// may have (the ticket buffer holds 2 + PWA_MAX_GROUPS counters: [0] finished
+// groups, [1] error flag, [2 + g] finished blocks of group g).
+#define PWA_GROUP 16
+#define PWA_MAX_GROUPS 4096
+
+// The last block (NT threads): rows[0 .. n) of `na` sums each -> entries
+// 0 .. na - 1 of out, the error flag as entry na.  Where NT / na >= 2 threads
+// are left per sum they take every so many rows each, so that the reads are
+// one round trip; then thread j adds their values in order.  Counters are
+// reset before the flag's entry: the host has every entry only after that.
+template <int NT>
+__device__ __forceinline__ void publish_rows(const double* __restrict__ rows, int n, int na,
+                                             unsigned int* __restrict__ ticket,
+                                             double* __restrict__ out, unsigned int seq) {
+  __shared__ double scratch[NT];
+  const int t = threadIdx.x, slices = NT / na;
+  if (slices >= 2) {
+    if (t < slices * na) {
+      const int j = t % na, s = t / na;
+      double a0 = 0.0, a1 = 0.0;
+      int r = s;
+#pragma unroll 4
+      for (; r + slices < n; r += 2 * slices) {
+        a0 += __ldcg(rows + (long long)r * na + j);
+        a1 += __ldcg(rows + (long long)(r + slices) * na + j);
+      }
+      if (r < n) a0 += __ldcg(rows + (long long)r * na + j);
+      scratch[t] = a0 + a1;
+    }
+    if (t == NT - 1) {
+      const unsigned int err = __ldcg(ticket + 1);
+      ticket[0] = 0u;
+      ticket[1] = 0u;
+      __threadfence();
+      ll_store(out, na, (double)err, seq);
+    }
+    __syncthreads();
+    if (t < na) {
+      double a = 0.0;
+      for (int s = 0; s < slices; ++s) a += scratch[s * na + t];
+      ll_store(out, t, a, seq);
+    }
+    return;
+  }
+  for (int j = t; j < na; j += NT) {
+    double a[4] = {0.0, 0.0, 0.0, 0.0};
+    int r = 0;
+#pragma unroll 4
+    for (; r + 4 <= n; r += 4)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) a[u] += __ldcg(rows + (long long)(r + u) * na + j);
+    for (; r < n; ++r) a[0] += __ldcg(rows + (long long)r * na + j);
+    ll_store(out, j, (a[0] + a[1]) + (a[2] + a[3]), seq);
+  }
+  if (t == NT - 1) {
+    const unsigned int err = __ldcg(ticket + 1);
+    ticket[0] = 0u;
+    ticket[1] = 0u;
+    __threadfence();
+    ll_store(out, na, (double)err, seq);
+  }
+}
+
+// Two levels (blocks of PWA_TPB threads; row b = block b's `na` sums, written
+// by its threads before the call): the last block of each group of PWA_GROUP
+// consecutive blocks sums the group's rows in block order into group row g,
+// stored after the block rows; the last group's block publishes the group
+// rows' sums.  *s_flag is a __shared__ int of the caller.
+// The tail of a launch is serial (row, counter, group row, counter, result):
+// counters that order by themselves instead of fences around them, the last
+// sum in one round trip of reads and entries that need no fence took a cached
+// evaluation of 5.5e3 events from 20.3 to 18.0 us, the plain one of 1.1e5
+// D -> K pi pi events from 23.1 to 20.3.
+__device__ __forceinline__ void grouped_publish(double* __restrict__ partials,
+                                                unsigned int* __restrict__ ticket, int na,
+                                                double* __restrict__ out, unsigned int seq,
+                                                int* s_flag) {
+  const int nb = (int)gridDim.x, g = (int)blockIdx.x / PWA_GROUP;
+  const int ng = (nb + PWA_GROUP - 1) / PWA_GROUP;
+  const int gs = min(PWA_GROUP, nb - g * PWA_GROUP);
+  double* grows = partials + (long long)nb * na;
+  __syncthreads();
+  if (threadIdx.x == 0) *s_flag = ticket_add(ticket + 2 + g) == (unsigned)gs - 1;
+  __syncthreads();
+  if (!*s_flag) return;
+  for (int j = threadIdx.x; j < na; j += PWA_TPB) {
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+    for (int r = 0; r < PWA_GROUP; ++r)
+      if (r < gs) s[r & 3] += __ldcg(partials + (long long)(g * PWA_GROUP + r) * na + j);
+    grows[(long long)g * na + j] = (s[0] + s[1]) + (s[2] + s[3]);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    ticket[2 + g] = 0u;
+    *s_flag = ticket_add(ticket) == (unsigned)ng - 1;
+  }
+  __syncthreads();
+  if (!*s_flag) return;
+  publish_rows<PWA_TPB>(grows, ng, na, ticket, out, seq);
+}
+
 template <typename R>
 __device__ __forceinline__ void eval_body(const Consts& C, const R* __restrict__ XA,
                                           const double* __restrict__ XM,
                                           const double* __restrict__ W, long long n_data,
                                           long long n_all, long long ld, int blocks_data,
-                                          double* __restrict__ partials) {
+                                          double* __restrict__ partials,
+                                          unsigned int* __restrict__ ticket,
+                                          double* __restrict__ out, unsigned int seq) {
   const bool is_data = (int)blockIdx.x < blocks_data;
   const long long beg = is_data ? 0 : n_data;
   const long long end = is_data ? n_data : n_all;
@@ -93,8 +202,20 @@ __device__ __forceinline__ void eval_body(const Consts& C, const R* __restrict__
     double s = 0.0;
 #pragma unroll
     for (int w2 = 0; w2 < PWA_TPB / 32; ++w2) s += red[w2][j];
-    partials[(long long)blockIdx.x * PWA_NACC + j] = s;
+    red[0][j] = s;
+    if (!ticket) partials[(long long)blockIdx.x * PWA_NACC + j] = s;
   }
+  if (!ticket) return;  // rows of PWA_NACC for pwa_reduce
+  // row of 2 PWA_NACC (a data block's sums in the first half, an MC block's
+  // in the second), reduced in the same launch
+  __syncthreads();
+  constexpr int NA2 = 2 * PWA_NACC;
+  for (int j = threadIdx.x; j < NA2; j += PWA_TPB) {
+    const int jj = j - (is_data ? 0 : PWA_NACC);
+    partials[(long long)blockIdx.x * NA2 + j] = jj >= 0 && jj < PWA_NACC ? red[0][jj] : 0.0;
+  }
+  __shared__ int s_last;
+  grouped_publish(partials, ticket, NA2, out, seq, &s_last);
 }
 
 // Blocks per SM the plain kernels are compiled for (register cap 65536 /
@@ -113,25 +234,24 @@ __device__ __forceinline__ void eval_body(const Consts& C, const R* __restrict__
 extern "C" __global__ void __launch_bounds__(PWA_TPB, PWA_EVAL_MINB)
     pwa_eval_f64(const Consts C, const double* __restrict__ XA, const double* __restrict__ XM,
                  const double* __restrict__ W, long long n_data, long long n_all, long long ld,
-                 int blocks_data, double* __restrict__ partials) {
-  eval_body<double>(C, XA, XM, W, n_data, n_all, ld, blocks_data, partials);
+                 int blocks_data, double* __restrict__ partials,
+                 unsigned int* __restrict__ ticket, double* __restrict__ out, unsigned int seq) {
+  eval_body<double>(C, XA, XM, W, n_data, n_all, ld, blocks_data, partials, ticket, out, seq);
 }
 
 extern "C" __global__ void __launch_bounds__(PWA_TPB, PWA_EVAL_MINB_F32)
     pwa_eval_f32(const Consts C, const float* __restrict__ XA, const double* __restrict__ XM,
                  const double* __restrict__ W, long long n_data, long long n_all, long long ld,
-                 int blocks_data, double* __restrict__ partials) {
-  eval_body<float>(C, XA, XM, W, n_data, n_all, ld, blocks_data, partials);
+                 int blocks_data, double* __restrict__ partials,
+                 unsigned int* __restrict__ ticket, double* __restrict__ out, unsigned int seq) {
+  eval_body<float>(C, XA, XM, W, n_data, n_all, ld, blocks_data, partials, ticket, out, seq);
 }
 
-// out[0..nacc) = data sums, out[nacc..2 nacc) = MC sums.  One warp per
-// accumulator; each lane strides over the blocks, then a fixed shuffle tree.
-// With seq_out set (out in mapped host memory), the call number seq is
-// written there last, after a system-scope fence that orders every warp's
-// out[] writes (observed through the block barrier) before it.
+// out[0..nacc) = data sums, out[nacc..2 nacc) = MC sums of the block rows
+// written without a ticket.  One warp per accumulator; each lane strides over
+// the blocks, then a fixed shuffle tree.
 extern "C" __global__ void pwa_reduce(const double* __restrict__ partials, int nacc,
-                                      int blocks_data, int nblocks, double* __restrict__ out,
-                                      double* __restrict__ seq_out, double seq) {
+                                      int blocks_data, int nblocks, double* __restrict__ out) {
   const int lane = threadIdx.x & 31;
   const int warps = blockDim.x >> 5;
   for (int j = (int)(threadIdx.x >> 5); j < 2 * nacc; j += warps) {
@@ -141,13 +261,6 @@ extern "C" __global__ void pwa_reduce(const double* __restrict__ partials, int n
     for (int b = b0 + lane; b < b1; b += 32) s += partials[(long long)b * nacc + jj];
     s = warp_sum(s);
     if (lane == 0) out[j] = s;
-  }
-  if (seq_out) {
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      __threadfence_system();
-      *seq_out = seq;
-    }
   }
 }
 
@@ -875,17 +988,9 @@ __device__ __forceinline__ void sc_issue(double* __restrict__ d, const float2* _
   if (half == 0) cp_async16(d + (PWA_NF + PWA_SC_NM) * PWA_TPB + col, W + s + c2);
 }
 
-// Ends with the ordered two-level reduction of pwa_eval_cached (grouped_sum,
-// declared below): block rows of 2 * PWA_NACC (a data block's sums in the
-// first half, an MC block's in the second); the last block writes the data
-// and MC sums to out[0 .. 2 PWA_NACC), the error flag and the call number
-// seq (publish_result); out may be mapped host memory.
-__device__ __forceinline__ bool grouped_sum(double* __restrict__ partials,
-                                            unsigned int* __restrict__ ticket, int na,
-                                            double* __restrict__ out, int* s_flag);
-__device__ __forceinline__ void publish_result(unsigned int* __restrict__ ticket, int na,
-                                               double* __restrict__ out, double seq);
-
+// Ends with the ordered two-level reduction (grouped_publish): block rows of
+// 2 * PWA_NACC (a data block's sums in the first half, an MC block's in the
+// second).
 // Bound: FP64 issue and latency (160 FP64 instructions per D -> K pi pi
 // event, one square root and one division per lineshape), then the launch
 // and the reduction's serial tail.  The columns' sums leave out what is
@@ -898,7 +1003,7 @@ extern "C" __global__ void __launch_bounds__(PWA_TPB, PWA_SC_MINB)
                         const double* __restrict__ XM, const double* __restrict__ W,
                         long long n_data, long long n_all, long long ld, int blocks_data,
                         double* __restrict__ partials, int smem_bytes,
-                        unsigned int* __restrict__ ticket, double* __restrict__ out, double seq) {
+                        unsigned int* __restrict__ ticket, double* __restrict__ out, unsigned int seq) {
   constexpr int K = PWA_NCOL, NS = PWA_NSRES > 0 ? PWA_NSRES : 1;
   const bool is_data = (int)blockIdx.x < blocks_data;
   const long long beg = is_data ? 0 : n_data;
@@ -1073,10 +1178,7 @@ extern "C" __global__ void __launch_bounds__(PWA_TPB, PWA_SC_MINB)
     }
     partials[(long long)blockIdx.x * NA2 + j] = sacc;
   }
-  __threadfence();
-  __syncthreads();
-  if (!grouped_sum(partials, ticket, NA2, out, &s_last)) return;
-  publish_result(ticket, NA2, out, seq);
+  grouped_publish(partials, ticket, NA2, out, seq, &s_last);
 }
 
 // Plain FP64 evaluation from the columns, where no mass or width is free (no
@@ -1160,7 +1262,7 @@ extern "C" __global__ void __launch_bounds__(PWA_TPB, EC_MINB)
     pwa_eval_cols(const Consts C, const double* __restrict__ XA, const double* __restrict__ XM,
                   const double* __restrict__ W, long long n_data, long long n_all, long long ld,
                   int blocks_data, double* __restrict__ partials,
-                  unsigned int* __restrict__ ticket, double* __restrict__ out, double seq) {
+                  unsigned int* __restrict__ ticket, double* __restrict__ out, unsigned int seq) {
 #if PWA_EVAL_COLS
   extern __shared__ __align__(16) double2 ec_smem[];
   double2* sF = ec_smem;                      // [PWA_NF][PWA_TPB]
@@ -1233,10 +1335,7 @@ extern "C" __global__ void __launch_bounds__(PWA_TPB, EC_MINB)
     const int jj = j - (is_data ? 0 : PWA_NACC);
     partials[(long long)blockIdx.x * NA2 + j] = jj >= 0 && jj < 1 + 2 * PWA_NCOL ? s_sum[jj] : 0.0;
   }
-  __threadfence();
-  __syncthreads();
-  if (!grouped_sum(partials, ticket, NA2, out, &s_last)) return;
-  publish_result(ticket, NA2, out, seq);
+  grouped_publish(partials, ticket, NA2, out, seq, &s_last);
 #endif
 }
 
@@ -1258,90 +1357,6 @@ __device__ __forceinline__ void stage_couplings(const CCoup& c, double* s_c) {
 #define PWA_STAGES 3
 #endif
 #define PWA_CACHE_NA (1 + 2 * PWA_NCOL)
-// Blocks per group of the two-level partial reduction, and the most groups
-// a launch may have (the ticket buffer holds 2 + PWA_MAX_GROUPS counters).
-#define PWA_GROUP 16
-#define PWA_MAX_GROUPS 4096
-
-// Sum of the block partials (rows of `na` doubles, one per block) by the
-// last block to finish: thread j owns accumulators j, j + PWA_TPB, ...,
-// reads the rows in order (a warp reads consecutive accumulators of a row:
-// coalesced) with four interleaved partial sums, so many loads are in
-// flight.  The order depends only on the row count: reproducible.
-__device__ __forceinline__ void last_block_sum(const double* __restrict__ partials, int nrows,
-                                               int na, double* __restrict__ out) {
-  for (int j = threadIdx.x; j < na; j += PWA_TPB) {
-    double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-    int b = 0;
-#pragma unroll 4
-    for (; b + 4 <= nrows; b += 4) {
-      s0 += __ldcg(partials + (long long)b * na + j);
-      s1 += __ldcg(partials + (long long)(b + 1) * na + j);
-      s2 += __ldcg(partials + (long long)(b + 2) * na + j);
-      s3 += __ldcg(partials + (long long)(b + 3) * na + j);
-    }
-    for (; b < nrows; ++b) s0 += __ldcg(partials + (long long)b * na + j);
-    out[j] = (s0 + s1) + (s2 + s3);
-  }
-}
-
-// Result publication by the block that wrote out[0 .. na): after the
-// block barrier, thread 0 writes the error flag, issues one system-scope
-// fence (cumulative: it orders the block's out[] writes, observed through
-// the barrier, before what follows) and writes the call number `seq` last,
-// so a host that sees out[na + 1] == seq (mapped memory) may read
-// everything before it.  Resets the counters for the next launch.
-__device__ __forceinline__ void publish_result(unsigned int* __restrict__ ticket, int na,
-                                               double* __restrict__ out, double seq) {
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    out[na] = (double)atomicOr((unsigned int*)(ticket + 1), 0u);
-    ticket[0] = 0u;
-    ticket[1] = 0u;
-    __threadfence_system();
-    out[na + 1] = seq;
-  }
-}
-
-// Ordered two-level reduction of the block partials (row b = block b's
-// `na` sums, written and fenced by every block before the call).  The last
-// block of each group of PWA_GROUP consecutive blocks (ticket[2 + g])
-// sums the group's rows in block order into group row g (stored after the
-// block rows); the last group (ticket[0]) sums the group rows in order into
-// out.  Returns true in that one block.  Counters are reset for the next
-// launch; the order depends only on the grid size, so results are
-// bitwise reproducible.  *s_flag is a __shared__ int of the caller.
-__device__ __forceinline__ bool grouped_sum(double* __restrict__ partials,
-                                            unsigned int* __restrict__ ticket, int na,
-                                            double* __restrict__ out, int* s_flag) {
-  const int nb = (int)gridDim.x, g = (int)blockIdx.x / PWA_GROUP;
-  const int ng = (nb + PWA_GROUP - 1) / PWA_GROUP;
-  const int gs = min(PWA_GROUP, nb - g * PWA_GROUP);
-  double* grows = partials + (long long)nb * na;
-  if (threadIdx.x == 0) *s_flag = (atomicAdd(ticket + 2 + g, 1u) == (unsigned)gs - 1);
-  __syncthreads();
-  if (!*s_flag) return false;
-  __threadfence();
-  for (int j = threadIdx.x; j < na; j += PWA_TPB) {
-    double s[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll
-    for (int r = 0; r < PWA_GROUP; ++r)
-      if (r < gs) s[r & 3] += __ldcg(partials + (long long)(g * PWA_GROUP + r) * na + j);
-    grows[(long long)g * na + j] = (s[0] + s[1]) + (s[2] + s[3]);
-  }
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    ticket[2 + g] = 0u;
-    *s_flag = (atomicAdd(ticket, 1u) == (unsigned)ng - 1);
-  }
-  __syncthreads();
-  if (!*s_flag) return false;
-  __threadfence();
-  last_block_sum(grows, ng, na, out);
-  return true;
-}
-
 // Persistent streaming kernel over the column cache.  Thread 0 keeps
 // PWA_STAGES tiles in flight with cp.async.bulk into a shared-memory ring
 // (full-barrier per stage with transaction bytes); every thread evaluates
@@ -1354,7 +1369,7 @@ __device__ __forceinline__ bool grouped_sum(double* __restrict__ partials,
 extern "C" __global__ void __launch_bounds__(PWA_TPB)
     pwa_eval_cached(const CCoup c, const float2* __restrict__ Fc, const double* __restrict__ Wc,
                     long long ntiles, double* __restrict__ partials,
-                    unsigned int* __restrict__ ticket, double* __restrict__ out, double seq) {
+                    unsigned int* __restrict__ ticket, double* __restrict__ out, unsigned int seq) {
   constexpr int NA = PWA_CACHE_NA;
   constexpr unsigned TILE_F = PWA_NF * PWA_TPB * sizeof(float2);
   constexpr unsigned TILE_W = PWA_TPB * sizeof(double);
@@ -1463,10 +1478,7 @@ extern "C" __global__ void __launch_bounds__(PWA_TPB)
     partials[(long long)blockIdx.x * NA + j] = s;
   }
   if (tid == 0 && s_err) atomicOr((unsigned int*)(ticket + 1), 1u);
-  __threadfence();
-  __syncthreads();
-  if (!grouped_sum(partials, ticket, NA, out, &s_last)) return;
-  publish_result(ticket, NA, out, seq);
+  grouped_publish(partials, ticket, NA, out, seq, &s_last);
 }
 
 // Direct-load variant of pwa_eval_cached: no shared-memory staging; each
@@ -1479,7 +1491,7 @@ extern "C" __global__ void __launch_bounds__(PWA_TPB, 4)
     pwa_eval_cached_direct(const CCoup c, const float2* __restrict__ Fc,
                            const double* __restrict__ Wc, long long ntiles,
                            double* __restrict__ partials, unsigned int* __restrict__ ticket,
-                           double* __restrict__ out, double seq) {
+                           double* __restrict__ out, unsigned int seq) {
   constexpr int NA = PWA_CACHE_NA;
   __shared__ double red[PWA_TPB / 32][NA];
   __shared__ int s_last;
@@ -1549,10 +1561,7 @@ extern "C" __global__ void __launch_bounds__(PWA_TPB, 4)
     for (int w2 = 0; w2 < PWA_TPB / 32; ++w2) s2 += red[w2][j];
     partials[(long long)blockIdx.x * NA + j] = s2;
   }
-  __threadfence();
-  __syncthreads();
-  if (!grouped_sum(partials, ticket, NA, out, &s_last)) return;
-  publish_result(ticket, NA, out, seq);
+  grouped_publish(partials, ticket, NA, out, seq, &s_last);
 }
 
 // ---------------------------------------------------------------------------
@@ -1722,7 +1731,7 @@ extern "C" __global__ void __launch_bounds__(PWA_TPB, PWA_WRED_MINB)
     pwa_eval_cached_wred(const CCoup c, const float2* __restrict__ Fc,
                          const double* __restrict__ Wc, long long ntiles,
                          double* __restrict__ partials, unsigned int* __restrict__ ticket,
-                         double* __restrict__ out, double seq) {
+                         double* __restrict__ out, unsigned int seq) {
   constexpr int NA = PWA_CACHE_NA;
   constexpr int NG = 2 * PWA_NCOL, MG = PWA_MG;
   __shared__ double red[PWA_TPB / 32][NA];
@@ -1764,10 +1773,7 @@ extern "C" __global__ void __launch_bounds__(PWA_TPB, PWA_WRED_MINB)
     for (int w2 = 0; w2 < PWA_TPB / 32; ++w2) s2 += red[w2][j];
     partials[(long long)blockIdx.x * NA + j] = s2;
   }
-  __threadfence();
-  __syncthreads();
-  if (!grouped_sum(partials, ticket, NA, out, &s_last)) return;
-  publish_result(ticket, NA, out, seq);
+  grouped_publish(partials, ticket, NA, out, seq, &s_last);
 }
 
 // ---------------------------------------------------------------------------
@@ -1787,7 +1793,7 @@ extern "C" __global__ void __launch_bounds__(PWA_TPB)
     pwa_eval_cached_ring2(const CCoup c, const float2* __restrict__ Fc,
                           const double* __restrict__ Wc, long long ntiles,
                           double* __restrict__ partials, unsigned int* __restrict__ ticket,
-                          double* __restrict__ out, double seq) {
+                          double* __restrict__ out, unsigned int seq) {
   constexpr int NA = PWA_CACHE_NA;
   constexpr int NG = 2 * PWA_NCOL, MG = PWA_GPAD / 32;
   constexpr unsigned TILE_F = PWA_NF * PWA_TPB * sizeof(float2);
@@ -1912,10 +1918,7 @@ extern "C" __global__ void __launch_bounds__(PWA_TPB)
     partials[(long long)blockIdx.x * NA + j] = s2;
   }
   if (tid == 0 && s_err) atomicOr((unsigned int*)(ticket + 1), 1u);
-  __threadfence();
-  __syncthreads();
-  if (!grouped_sum(partials, ticket, NA, out, &s_last)) return;
-  publish_result(ticket, NA, out, seq);
+  grouped_publish(partials, ticket, NA, out, seq, &s_last);
 }
 
 // ---------------------------------------------------------------------------
@@ -1928,8 +1931,8 @@ extern "C" __global__ void __launch_bounds__(PWA_TPB)
 // the error flag set -- what a stalled ring kernel reports.
 extern "C" __global__ void __launch_bounds__(PWA_TPB)
     pwa_wait_check(const double* __restrict__ src, unsigned polls,
-                   unsigned int* __restrict__ ticket, double* __restrict__ out, double seq,
-                   int na) {
+                   unsigned int* __restrict__ ticket, double* __restrict__ out,
+                   unsigned int seq, int na) {
   __shared__ __align__(128) double buf[PWA_TPB];
   __shared__ __align__(8) unsigned long long never, real;
   if (threadIdx.x == 0) {
@@ -1946,59 +1949,24 @@ extern "C" __global__ void __launch_bounds__(PWA_TPB)
     mbar_wait(&real, 0u, PWA_WAIT_LIMIT);
     if (!ok) atomicOr((unsigned int*)(ticket + 1), 1u);
   }
-  for (int j = threadIdx.x; j < na; j += PWA_TPB) out[j] = 0.0;
-  publish_result(ticket, na, out, seq);
+  __syncthreads();
+  // the sums of no rows: zeros, and the error flag
+  publish_rows<PWA_TPB>(src, 0, na, ticket, out, seq);
 }
 
 // ---------------------------------------------------------------------------
 // Kernels with one block per SM.  Their block partials are few (one row per
-// SM), so a single ordered level replaces the two-level reduction: every
-// block writes its row and fences it, the last block to take ticket[0] sums
-// all rows.  Its threads form `slices` = blockDim / na groups; slice s sums
-// rows s, s + slices, ... in order (two interleaved chains), then thread j
-// adds the slices' values in order.  The order depends only on the grid:
-// bitwise reproducible.  scratch: __shared__, at least blockDim doubles.
-__device__ __forceinline__ bool flat_sum(const double* __restrict__ partials,
-                                         unsigned int* __restrict__ ticket, int na,
-                                         double* __restrict__ out, double* scratch,
-                                         int* s_flag) {
-  const int nrows = (int)gridDim.x, nt = (int)blockDim.x, t = (int)threadIdx.x;
-  if (t == 0) *s_flag = (atomicAdd(ticket, 1u) == (unsigned)nrows - 1);
+// SM), so a single ordered level replaces the two-level reduction: the last
+// block to take ticket[0] publishes the sums of all rows.
+template <int NT>
+__device__ __forceinline__ void flat_publish(const double* __restrict__ partials,
+                                             unsigned int* __restrict__ ticket, int na,
+                                             double* __restrict__ out, unsigned int seq,
+                                             int* s_flag) {
   __syncthreads();
-  if (!*s_flag) return false;
-  __threadfence();
-  const int slices = nt / na;
-  if (slices == 0) {
-    for (int j = t; j < na; j += nt) {
-      double a0 = 0.0, a1 = 0.0;
-      int r = 0;
-      for (; r + 1 < nrows; r += 2) {
-        a0 += __ldcg(partials + (long long)r * na + j);
-        a1 += __ldcg(partials + (long long)(r + 1) * na + j);
-      }
-      if (r < nrows) a0 += __ldcg(partials + (long long)r * na + j);
-      out[j] = a0 + a1;
-    }
-    return true;
-  }
-  if (t < slices * na) {
-    const int j = t % na, s = t / na;
-    double a0 = 0.0, a1 = 0.0;
-    int r = s;
-    for (; r + slices < nrows; r += 2 * slices) {
-      a0 += __ldcg(partials + (long long)r * na + j);
-      a1 += __ldcg(partials + (long long)(r + slices) * na + j);
-    }
-    if (r < nrows) a0 += __ldcg(partials + (long long)r * na + j);
-    scratch[s * na + j] = a0 + a1;
-  }
+  if (threadIdx.x == 0) *s_flag = ticket_add(ticket) == gridDim.x - 1;
   __syncthreads();
-  for (int j = t; j < na; j += nt) {
-    double a = 0.0;
-    for (int s = 0; s < slices; ++s) a += scratch[s * na + j];
-    out[j] = a;
-  }
-  return true;
+  if (*s_flag) publish_rows<NT>(partials, (int)gridDim.x, na, ticket, out, seq);
 }
 
 // Warp sums of one block (acc0 on every lane, column group m's entry on
@@ -2025,8 +1993,6 @@ __device__ __forceinline__ void cached_block_row(double acc0, const double* accg
     for (int w2 = 0; w2 < NW; ++w2) s += red[w2][j];
     partials[(long long)blockIdx.x * NA + j] = s;
   }
-  __threadfence();
-  __syncthreads();
 }
 
 // Variant 4: one block of PWA_WIDE_WARPS warps per SM.  Each warp streams a
@@ -2041,12 +2007,11 @@ extern "C" __global__ void __launch_bounds__(PWA_WIDE_WARPS * 32, 1)
     pwa_eval_cached_wide(const CCoup c, const float2* __restrict__ Fc,
                          const double* __restrict__ Wc, long long ntiles,
                          double* __restrict__ partials, unsigned int* __restrict__ ticket,
-                         double* __restrict__ out, double seq) {
+                         double* __restrict__ out, unsigned int seq) {
   constexpr int NA = PWA_CACHE_NA, MG = PWA_MG;
   constexpr int NW = PWA_WIDE_WARPS, UPT = PWA_TPB / 32;
   __shared__ double red[NW][NA];
   __shared__ double s_c[2 * PWA_NCOL];
-  __shared__ double scratch[NW * 32];
   __shared__ int s_last;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   stage_couplings(c, s_c);
@@ -2074,8 +2039,7 @@ extern "C" __global__ void __launch_bounds__(PWA_WIDE_WARPS * 32, 1)
     for (int m = 0; m < MG; ++m) accg[m] += (double)gs[m];
   }
   cached_block_row<NW>(acc0, accg, red, warp, lane, true, partials);
-  if (!flat_sum(partials, ticket, NA, out, scratch, &s_last)) return;
-  publish_result(ticket, NA, out, seq);
+  flat_publish<NW * 32>(partials, ticket, NA, out, seq, &s_last);
 }
 
 // Variant 5: warp-specialised ring, one block per SM.  One producer lane
@@ -2102,7 +2066,7 @@ extern "C" __global__ void __launch_bounds__(PWA_TMA_THREADS, 1)
     pwa_eval_cached_tma(const CCoup c, const float2* __restrict__ Fc,
                         const double* __restrict__ Wc, long long ntiles,
                         double* __restrict__ partials, unsigned int* __restrict__ ticket,
-                        double* __restrict__ out, double seq, int stages) {
+                        double* __restrict__ out, unsigned int seq, int stages) {
   constexpr int NA = PWA_CACHE_NA, MG = PWA_MG;
   constexpr int UPT = PWA_TPB / 32, NCW = PWA_TMA_GROUPS * UPT;
   constexpr unsigned TILE_F = PWA_NF * PWA_TPB * sizeof(float2);
@@ -2112,7 +2076,6 @@ extern "C" __global__ void __launch_bounds__(PWA_TMA_THREADS, 1)
   __shared__ __align__(8) unsigned long long full[PWA_TMA_MAXST], empty[PWA_TMA_MAXST];
   __shared__ double red[NCW][NA];
   __shared__ double s_c[2 * PWA_NCOL];
-  __shared__ double scratch[PWA_TMA_THREADS];
   __shared__ int s_last;
   __shared__ volatile int s_err;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -2120,10 +2083,7 @@ extern "C" __global__ void __launch_bounds__(PWA_TMA_THREADS, 1)
     // refused depth: report it like a stalled ring (zero sums, error flag)
     if (tid == 0) atomicOr((unsigned int*)(ticket + 1), 1u);
     for (int j = tid; j < NA; j += PWA_TMA_THREADS) partials[(long long)blockIdx.x * NA + j] = 0.0;
-    __threadfence();
-    __syncthreads();
-    if (!flat_sum(partials, ticket, NA, out, scratch, &s_last)) return;
-    publish_result(ticket, NA, out, seq);
+    flat_publish<PWA_TMA_THREADS>(partials, ticket, NA, out, seq, &s_last);
     return;
   }
   if (tid == 0) {
@@ -2192,8 +2152,7 @@ extern "C" __global__ void __launch_bounds__(PWA_TMA_THREADS, 1)
     atomicOr((unsigned int*)(ticket + 1), 1u);
   }
   cached_block_row<NCW>(acc0, accg, red, warp, lane, warp < NCW, partials);
-  if (!flat_sum(partials, ticket, NA, out, scratch, &s_last)) return;
-  publish_result(ticket, NA, out, seq);
+  flat_publish<PWA_TMA_THREADS>(partials, ticket, NA, out, seq, &s_last);
 }
 
 // ---------------------------------------------------------------------------
@@ -2699,7 +2658,7 @@ extern "C" __global__ void __launch_bounds__(PWA_TPB, PWA_MULTI_MINB)
     pwa_eval_multi(const long long* __restrict__ meta, int n_req, long long n_chunks,
                    long long n_tiles, long long n_groups, const float2* __restrict__ Fc,
                    const double* __restrict__ Wc, double* __restrict__ rows,
-                   unsigned int* __restrict__ count, double* __restrict__ out, double seq) {
+                   unsigned int* __restrict__ count, double* __restrict__ out, unsigned int seq) {
   constexpr int NA = PWA_CACHE_NA, NG = 2 * PWA_NCOL, MG = PWA_MG, NW = PWA_TPB / 32;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const MultiMeta m(meta, n_req);
@@ -2796,7 +2755,7 @@ extern "C" __global__ void __launch_bounds__(PWA_TPB, PWA_MULTI_MINB)
         if (atomicAdd(count + n_groups + n_req, 1u) == (unsigned)n_req - 1) {
           count[n_groups + n_req] = 0u;
           __threadfence_system();
-          out[(long long)n_req * NA] = seq;
+          out[(long long)n_req * NA] = (double)seq;
         }
       }
       __syncwarp();

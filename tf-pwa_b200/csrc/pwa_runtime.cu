@@ -94,7 +94,8 @@ struct pwa_plan {
   double* d_map = nullptr;         // its device address
   double* h_map_sc = nullptr;      // mapped result of pwa_eval_shapecache (2 nacc + 2)
   double* d_map_sc = nullptr;
-  double seq = 0.0;
+  unsigned int seq = 0;          // number of the last call with a mapped result, never 0 after one
+  std::vector<double> sums;      // the last such result and its error flag
   std::vector<double> gram;  // MC Gram matrix, (re, im) row-major ncol x ncol
   bool gram_valid = false;
   int gram_method = -1;  // 0 FP64 CUDA cores, 1 tensor cores, -1 automatic (0)
@@ -156,6 +157,11 @@ struct pwa_plan {
 };
 
 namespace {
+
+unsigned int next_seq(pwa_plan* h) {
+  if (++h->seq == 0) ++h->seq;
+  return h->seq;
+}
 
 // message of the last failed call without a plan handle (per host thread)
 thread_local std::string g_err;
@@ -482,8 +488,9 @@ int pwa_plan_create(const char* src, size_t src_len, int n_mass, int n_angle, in
   CU(cudaMalloc(&h->ticket, kTicketWords * sizeof(unsigned int)));
   CU(cudaMemset(h->ticket, 0, kTicketWords * sizeof(unsigned int)));
   {
-    const size_t b0 = (sizeof(double) * (2 * ncol + 4) + 255) / 256 * 256;
-    h->pin_batch = b0 + (sizeof(double) * (2 * h->nacc + 2) + 255) / 256 * 256;
+    // two words per entry (ll_store): sums and the error flag
+    const size_t b0 = (16 * (size_t)(2 * ncol + 2) + 255) / 256 * 256;
+    h->pin_batch = b0 + (16 * (size_t)(2 * h->nacc + 1) + 255) / 256 * 256;
     h->pin_batch_cap = 256 * 1024;
     CU(cudaHostAlloc(&h->h_pin, h->pin_batch + h->pin_batch_cap, cudaHostAllocMapped));
     CU(cudaHostGetDevicePointer((void**)&h->d_pin, h->h_pin, 0));
@@ -493,9 +500,8 @@ int pwa_plan_create(const char* src, size_t src_len, int n_mass, int n_angle, in
     h->d_map_sc = (double*)(h->d_pin + b0);
   }
   // no call number yet: pinned memory may come back from a closed plan with
-  // that plan's last number in it
-  h->h_map[2 * ncol + 2] = -1.0;
-  h->h_map_sc[2 * h->nacc + 1] = -1.0;
+  // that plan's numbers in it
+  std::memset(h->h_pin, 0, h->pin_batch);
   return PWA_OK;
 }
 
@@ -584,7 +590,8 @@ int pwa_upload_events(pwa_plan* h, const double* xm, const double* xa, const dou
   CU(grid(h->k.eval_f64, &h->nblocks, &h->blocks_data));
   CU(grid(h->k.eval_f32, &h->nblocks32, &h->blocks_data32));
   const int nb_max = h->nblocks > h->nblocks32 ? h->nblocks : h->nblocks32;
-  int rc = ensure_partials(h, (long long)nb_max * h->nacc);
+  // block rows of 2 nacc and the group rows of the in-kernel reduction
+  int rc = ensure_partials(h, (long long)(nb_max + (nb_max + 15) / 16) * 2 * h->nacc);
   if (rc) return rc;
   CU(cudaStreamSynchronize(s));
   return PWA_OK;
@@ -607,40 +614,55 @@ int pwa_eval_enqueue(pwa_plan* h, const double* consts, int precision, int mc, v
   int bd = mc ? nb_data : nblocks;
   const void* xa = precision == PWA_PLAIN_F64 ? (const void*)h->xa : (const void*)h->xa32;
   long long nd = h->n_data, ld = h->ld;
-  void* args[] = {cbuf.data(), (void*)&xa, &h->xm, &h->w, &nd, &n_all, &ld, &bd, &h->partials};
-  int rc = launch(h, precision == PWA_PLAIN_F64 ? h->k.eval_f64 : h->k.eval_f32, dim3(nblocks),
-                  dim3(h->tpb), args, s);
-  if (rc) return rc;
-  int nacc = h->nacc;
   // sums into the mapped result (with mc = 0 the MC half comes out zero:
-  // no MC blocks), the call number last
-  h->seq += 1.0;
-  double seq = h->seq;
-  double* seq_out = h->d_map_sc + 2 * nacc + 1;
-  void* args2[] = {&h->partials, &nacc, &bd, &nblocks, &h->d_map_sc, &seq_out, &seq};
-  return launch(h, h->k.reduce, dim3(1), dim3(1024), args2, s);
+  // no MC blocks)
+  unsigned int seq = next_seq(h);
+  void* args[] = {cbuf.data(), (void*)&xa, &h->xm, &h->w, &nd, &n_all, &ld, &bd, &h->partials,
+                  &h->ticket, &h->d_map_sc, &seq};
+  return launch(h, precision == PWA_PLAIN_F64 ? h->k.eval_f64 : h->k.eval_f32, dim3(nblocks),
+                dim3(h->tpb), args, s);
 }
 
 namespace {
-// Wait for the sums of the last pwa_eval_enqueue / pwa_eval_shapecache_enqueue
-// in the mapped result (its call number is written last); after 1 s without
-// it, synchronise the stream (which also surfaces launch errors).
-int wait_mapped_sums(pwa_plan* h, cudaStream_t s) {
-  const int na2 = 2 * h->nacc;
-  const volatile double* m = h->h_map_sc;
+// The n entries of the call numbered h->seq from a mapped result (ll_store:
+// two 8-byte words per entry, the number in each word's upper half) into
+// h->sums.  After limit_s seconds without one of them (a failed launch or a
+// very long kernel), synchronise the stream, which also surfaces launch
+// errors, and look once more; false when the result is not there then.
+bool wait_result(pwa_plan* h, const double* mapped, int n, cudaStream_t s, double limit_s) {
+  const volatile unsigned long long* m = (const volatile unsigned long long*)mapped;
+  const unsigned long long seq = h->seq;
+  h->sums.resize(n);
   const auto t0 = std::chrono::steady_clock::now();
-  for (unsigned it = 1; m[na2 + 1] != h->seq; ++it) {
-    if ((it & 4095u) == 0 &&
-        std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count() > 1.0) {
-      CU(cudaStreamSynchronize(s));
-      break;
+  bool late = false;
+  unsigned it = 0;
+  for (int j = 0; j < n; ++j) {
+    unsigned long long lo = m[2 * j], hi = m[2 * j + 1];
+    while (lo >> 32 != seq || hi >> 32 != seq) {
+      if (late) return false;
+      if ((++it & 4095u) == 0 &&
+          std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count() > limit_s) {
+        cudaStreamSynchronize(s);
+        late = true;
+      }
+      lo = m[2 * j];
+      hi = m[2 * j + 1];
     }
+    const unsigned long long b = (lo & 0xffffffffull) | (hi << 32);
+    std::memcpy(&h->sums[j], &b, sizeof(double));
   }
-  std::atomic_thread_fence(std::memory_order_acquire);
-  if (m[na2 + 1] != h->seq) {
+  return true;
+}
+
+// The data and MC sums of the last plain, FP32 or floating-shape evaluation.
+int wait_mapped_sums(pwa_plan* h, cudaStream_t s, double* out) {
+  const int na2 = 2 * h->nacc;
+  if (!wait_result(h, h->h_map_sc, na2 + 1, s, 1.0)) {
     cudaMemset(h->ticket, 0, kTicketWords * sizeof(unsigned int));
     return set_err(h, PWA_ERR_CUDA, "evaluation did not complete (stale result)");
   }
+  if (h->sums[na2] != 0.0) return set_err(h, PWA_ERR_CUDA, "evaluation: error flag set");
+  std::copy(h->sums.begin(), h->sums.begin() + na2, out);
   return PWA_OK;
 }
 }  // namespace
@@ -679,19 +701,14 @@ int eval_cols(pwa_plan* h, const double* consts, cudaStream_t s, double* out) {
   }
   std::vector<double> cbuf = consts_block(h, consts);
   long long nd = h->n_data, na = h->n_data + h->n_mc, ld = h->ld;
-  h->seq += 1.0;
-  double seq = h->seq;
+  unsigned int seq = next_seq(h);
   void* args[] = {cbuf.data(), &h->xa, &h->xm, &h->w, &nd, &na, &ld, &h->ec_blocks_data,
                   &h->partials, &h->ticket, &h->d_map_sc, &seq};
   cudaError_t e = cudaLaunchKernel((const void*)h->k.eval_cols, dim3(h->ec_blocks), dim3(h->tpb),
                                    args, (size_t)h->ec_smem, s);
   if (e != cudaSuccess)
     return set_err(h, PWA_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e));
-  int rc = wait_mapped_sums(h, s);
-  if (rc) return rc;
-  const volatile double* m = h->h_map_sc;
-  for (int j = 0; j < 2 * h->nacc; ++j) out[j] = m[j];
-  return PWA_OK;
+  return wait_mapped_sums(h, s, out);
 }
 
 // Whether no trainable variable takes a derivative through the kernels'
@@ -707,13 +724,10 @@ int pwa_eval(pwa_plan* h, const double* consts, int precision, int mc, void* str
   if (!out) return set_err(h, PWA_ERR_ARG, "null output");
   int rc = pwa_eval_enqueue(h, consts, precision, mc, stream);
   if (rc) return rc;
-  rc = wait_mapped_sums(h, (cudaStream_t)stream);
+  rc = wait_mapped_sums(h, (cudaStream_t)stream, out);
   if (rc) return rc;
-  const int nacc = h->nacc;
-  const volatile double* m = h->h_map_sc;
-  for (int j = 0; j < 2 * nacc; ++j) out[j] = m[j];
   if (!mc)
-    for (int j = 0; j < nacc; ++j) out[nacc + j] = 0.0;
+    for (int j = 0; j < h->nacc; ++j) out[h->nacc + j] = 0.0;
   return PWA_OK;
 }
 
@@ -783,8 +797,7 @@ int pwa_eval_shapecache_enqueue(pwa_plan* h, const double* consts, const double*
   }
   long long nd = h->n_data, na = h->n_data + h->n_mc, ld = h->ld;
   int bd = h->sc_blocks_data, nb = h->sc_blocks, smem = h->sc_smem;
-  h->seq += 1.0;
-  double seq = h->seq;
+  unsigned int seq = next_seq(h);
   void* args[] = {cbuf.data(), rbuf.data(), &h->scache, &h->xm, &h->w, &nd, &na, &ld, &bd,
                   &h->partials, &smem, &h->ticket, &h->d_map_sc, &seq};
   cudaError_t e = cudaLaunchKernel((const void*)h->k.eval_shapecache, dim3(nb), dim3(h->tpb), args,
@@ -800,15 +813,7 @@ int pwa_eval_shapecache(pwa_plan* h, const double* consts, const double* ratio, 
   if (!out) return set_err(h, PWA_ERR_ARG, "null output");
   int rc = pwa_eval_shapecache_enqueue(h, consts, ratio, stream);
   if (rc) return rc;
-  // the kernel publishes its call number last (after a system fence) into
-  // the mapped result
-  rc = wait_mapped_sums(h, (cudaStream_t)stream);
-  if (rc) return rc;
-  const int na2 = 2 * h->nacc;
-  const volatile double* m = h->h_map_sc;
-  if (m[na2] != 0.0) return set_err(h, PWA_ERR_CUDA, "floating-shape evaluation: error flag set");
-  for (int j = 0; j < na2; ++j) out[j] = m[j];
-  return PWA_OK;
+  return wait_mapped_sums(h, (cudaStream_t)stream, out);
 }
 
 int pwa_eval_pdf(pwa_plan* h, const double* consts, int precision, long long beg, long long end,
@@ -1227,8 +1232,7 @@ int pwa_eval_cached_enqueue(pwa_plan* h, const double* ck, void* stream) {
   cudaStream_t s = (cudaStream_t)stream;
   std::vector<double> cbuf(ck, ck + 2 * h->ncol);
   long long nt = h->ntiles;
-  h->seq += 1.0;
-  double seq = h->seq;
+  unsigned int seq = next_seq(h);
   void* args[] = {cbuf.data(), &h->fcache, &h->wcache, &nt, &h->partials, &h->ticket, &h->d_map,
                   &seq, &h->tma_stages};
   int variant = h->cached_variant >= 0 ? h->cached_variant : 2;
@@ -1257,39 +1261,17 @@ int pwa_eval_cached_enqueue(pwa_plan* h, const double* ck, void* stream) {
   return PWA_OK;
 }
 
-// Wait for the last cached launch: the kernel publishes its call number
-// last (after system fences) into mapped host memory, so polling it returns
-// as soon as the sums are visible, without a stream synchronisation.  After
-// `limit_s` seconds without it (a failed launch or a very long kernel) fall
-// back to synchronising the stream, which also surfaces launch errors.
-void wait_cached(pwa_plan* h, cudaStream_t s, double limit_s = 1.0) {
+// Sums of the last cached launch (1 + 2 ncol of them), polled from mapped
+// host memory without a stream synchronisation.
+int cached_result(pwa_plan* h, cudaStream_t s, const double** sums, double limit_s = 1.0) {
   const int na = 1 + 2 * h->ncol;
-  const volatile double* m = h->h_map;
-  const auto t0 = std::chrono::steady_clock::now();
-  for (unsigned it = 1;; ++it) {
-    if (m[na + 1] == h->seq) {
-      std::atomic_thread_fence(std::memory_order_acquire);
-      return;
-    }
-    if ((it & 4095u) == 0 &&
-        std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count() > limit_s) {
-      cudaStreamSynchronize(s);
-      return;
-    }
-  }
-}
-
-// Result of the last cached launch (after the stream has been synchronised):
-// checks the error flag and the call number.
-int cached_result(pwa_plan* h, const double** sums) {
-  const int na = 1 + 2 * h->ncol;
-  const volatile double* m = h->h_map;
-  if (m[na + 1] != h->seq) {
+  if (!wait_result(h, h->h_map, na + 1, s, limit_s)) {
     cudaMemset(h->ticket, 0, kTicketWords * sizeof(unsigned int));
     return set_err(h, PWA_ERR_CUDA, "cached evaluation did not complete (stale result)");
   }
-  if (m[na] != 0.0) return set_err(h, PWA_ERR_CUDA, "cached evaluation: a barrier wait timed out");
-  *sums = h->h_map;
+  if (h->sums[na] != 0.0)
+    return set_err(h, PWA_ERR_CUDA, "cached evaluation: a barrier wait timed out");
+  *sums = h->sums.data();
   return PWA_OK;
 }
 
@@ -1299,19 +1281,17 @@ int pwa_wait_check(pwa_plan* h, int mode, unsigned polls, double host_limit_s, v
   if ((mode != 0 && mode != 1) || !(host_limit_s > 0.0) || polls < 1)
     return set_err(h, PWA_ERR_ARG, "invalid wait-check arguments");
   cudaStream_t s = (cudaStream_t)stream;
-  h->seq += 1.0;
+  unsigned int seq = next_seq(h);
   if (mode == 0) {
     // any 1 KB of device memory serves as the source of the one real copy
     const double* src = (const double*)h->ticket;
     int na = 1 + 2 * h->ncol;
-    double seq = h->seq;
     void* args[] = {(void*)&src, &polls, &h->ticket, &h->d_map, &seq, &na};
     const int rc = launch(h, h->k.wait_check, dim3(1), dim3(h->tpb), args, s);
     if (rc) return rc;
   }
-  wait_cached(h, s, host_limit_s);
   const double* sd = nullptr;
-  return cached_result(h, &sd);
+  return cached_result(h, s, &sd, host_limit_s);
 }
 
 int pwa_fma_peak(pwa_plan* h, int precision, long long iters, void* stream, double* out) {
@@ -1430,9 +1410,8 @@ int pwa_autotune_cached(pwa_plan* h, const double* ck, int reps, void* stream, i
                                         "): " + cudaGetErrorString(e));
       break;
     }
-    wait_cached(h, s);
     const double* sd = nullptr;
-    rc = cached_result(h, &sd);
+    rc = cached_result(h, s, &sd);
     if (rc) break;
     const double us = 1e3 * ms / reps;
     out[c] = us;
@@ -1643,9 +1622,8 @@ int pwa_pieces_cached(pwa_plan* h, const double* vars, double sw, double mc_shar
   int rc = pwa_eval_cached_enqueue(h, ck.data(), stream);
   if (rc) return rc;
   const int rc2 = pieces_before(h, z.data(), ph.data(), ck.data(), sw, mc_share, J.data(), out);
-  wait_cached(h, s);
   const double* sd = nullptr;
-  rc = cached_result(h, &sd);
+  rc = cached_result(h, s, &sd);
   if (rc) return rc;
   if (rc2) return rc2;
   pieces_after(h, J.data(), sd, out);
@@ -1832,8 +1810,7 @@ int pwa_pieces_multi(pwa_plan* h, int n_req, const long long* first_tile, const 
   if (h->multi_bps > 0 && h->multi_bps < per_sm) per_sm = h->multi_bps;
   long long nb = (long long)per_sm * h->sms;
   if (nb > n_chunks) nb = n_chunks;
-  h->seq += 1.0;
-  double seq = h->seq;
+  unsigned int seq = next_seq(h);
   const volatile double* mark = h_res + (size_t)n_req * NA;
   h_res[(size_t)n_req * NA] = -1.0;  // the mark's place follows the request count
   void* a1[] = {&d_meta, &n_req, &n_chunks, &n_work, &n_groups, &h->pool_f, &h->pool_w,
@@ -1846,14 +1823,14 @@ int pwa_pieces_multi(pwa_plan* h, int n_req, const long long* first_tile, const 
     rc = pieces_before(h, &zs[nc * r], &phs[nc * r], ck + 2 * K * (size_t)r, sw[r], mc_share,
                        J.data() + h->jac.size() * r, out + (size_t)r * (3 + 2 * P));
   const auto w0 = std::chrono::steady_clock::now();
-  for (unsigned it = 1; *mark != seq; ++it)
+  for (unsigned it = 1; *mark != (double)seq; ++it)
     if ((it & 4095u) == 0 &&
         std::chrono::duration<double>(std::chrono::steady_clock::now() - w0).count() > 1.0) {
       CU(cudaStreamSynchronize(s));
       break;
     }
   std::atomic_thread_fence(std::memory_order_acquire);
-  if (*mark != seq) {
+  if (*mark != (double)seq) {
     cudaMemset(d_count, 0, sizeof(unsigned int) * h->mcount_cap);
     return set_err(h, PWA_ERR_CUDA, "batch evaluation did not complete (stale result)");
   }
@@ -2574,14 +2551,15 @@ extern "C" int pwa_eval_noalloc(pwa_plan* h, const double* consts, const double*
   cudaStream_t s = (cudaStream_t)stream;
   std::vector<double> cbuf = consts_block(h, consts);
   long long n_all = n;
+  // no ticket: block rows only
+  unsigned int *no_ticket = nullptr, no_seq = 0;
+  double* no_out = nullptr;
   void* args[] = {cbuf.data(), (void*)&xa, (void*)&xm, (void*)&w, &n_data, &n_all, &ld,
-                  &blocks_data, &scratch};
+                  &blocks_data, &scratch, &no_ticket, &no_out, &no_seq};
   rc = launch(h, h->k.eval_f64, dim3(nblocks), dim3(h->tpb), args, s);
   if (rc) return rc;
   int nacc = h->nacc;
-  double* no_seq = nullptr;
-  double seq0 = 0.0;
-  void* args2[] = {&scratch, &nacc, &blocks_data, &nblocks, &out, &no_seq, &seq0};
+  void* args2[] = {&scratch, &nacc, &blocks_data, &nblocks, &out};
   return launch(h, h->k.reduce, dim3(1), dim3(1024), args2, s);
 }
 
