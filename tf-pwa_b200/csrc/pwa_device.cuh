@@ -253,26 +253,6 @@ __device__ __forceinline__ float warp_sum_entries(const float (&v)[C], int lane)
   }
 }
 
-// --------------------------------------------------- results to the host
-// Entry j of a result in mapped host memory: the two halves of v as two
-// 8-byte words, each with the call's number in its upper half.  An 8-byte
-// store is whole, so the host takes an entry when both words carry the
-// number it waits for: no fence and no mark written last.
-__device__ __forceinline__ void ll_store(double* out, int j, double v, unsigned int seq) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(v);
-  const unsigned long long s = (unsigned long long)seq << 32;
-  asm volatile("st.volatile.global.v2.u64 [%0], {%1, %2};" ::"l"(out + 2 * j),
-               "l"(s | (b & 0xffffffffull)), "l"(s | (b >> 32))
-               : "memory");
-}
-// counter increment that orders the block's writes before it (after a block
-// barrier) and the reads after it (before one)
-__device__ __forceinline__ unsigned int ticket_add(unsigned int* p) {
-  unsigned int old;
-  asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(old) : "l"(p) : "memory");
-  return old;
-}
-
 // clip_log and its derivative in FP64
 __device__ __forceinline__ double clip_log(double x, double* dx) {
   const double eps = 1e-6;

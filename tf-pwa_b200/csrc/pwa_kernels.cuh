@@ -44,6 +44,25 @@
 #define PWA_GROUP 16
 #define PWA_MAX_GROUPS 4096
 
+// Entry j of a result in mapped host memory: the two halves of v as two
+// 8-byte words, each with the call's number in its upper half.  An 8-byte
+// store is whole, so the host takes an entry when both words carry the
+// number it waits for: no fence and no mark written last.
+__device__ __forceinline__ void ll_store(double* out, int j, double v, unsigned int seq) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+  const unsigned long long s = (unsigned long long)seq << 32;
+  asm volatile("st.volatile.global.v2.u64 [%0], {%1, %2};" ::"l"(out + 2 * j),
+               "l"(s | (b & 0xffffffffull)), "l"(s | (b >> 32))
+               : "memory");
+}
+// counter increment that orders the block's writes before it (after a block
+// barrier) and the reads after it (before one)
+__device__ __forceinline__ unsigned int ticket_add(unsigned int* p) {
+  unsigned int old;
+  asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(old) : "l"(p) : "memory");
+  return old;
+}
+
 // The last block (NT threads): rows[0 .. n) of `na` sums each -> entries
 // 0 .. na - 1 of out, the error flag as entry na.  Where NT / na >= 2 threads
 // are left per sum they take every so many rows each, so that the reads are
