@@ -19,6 +19,7 @@ per event in ``dat_order`` (``tf_pwa/data.py:300-365``); an index matching
 Every evaluation runs on the CUDA engine; there is no CPU path.
 """
 import json
+import operator
 import os
 import re
 import time
@@ -281,16 +282,23 @@ class FCN:
         elif len(x):
             self.vm.set_all(list(x))
 
+    _getter = None
+
+    def _values(self):
+        """Every variable's value in layout order."""
+        if self._getter is None:
+            n = self._var_names
+            self._getter = operator.itemgetter(*n) if len(n) > 1 else lambda v: (v[n[0]],)
+        return self._getter(self.vm.variables)
+
     def get_nll_grad(self, x=None):
         self._set(x)
         if self.vm.trainable_vars != self._train:
             self._relayout()
         if self.use_gram:
-            v = self.vm.variables
-            nll, g = self.eng.nll_grad_cached([v[k] for k in self._var_names])
+            nll, g = self.eng.nll_grad_cached(self._values())
         elif self.native_host:
-            v = self.vm.variables
-            nll, g = self.eng.nll_grad_vars([v[k] for k in self._var_names], self._form)
+            nll, g = self.eng.nll_grad_vars(self._values(), self._form)
         else:
             nll, g = self.eng.nll_grad(self.vm.get_all_dic(), self.vm.trainable_vars,
                                        self.precision)

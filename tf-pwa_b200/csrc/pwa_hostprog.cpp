@@ -463,6 +463,17 @@ bool parse(const int* ip, long long n_ip, const double* dp, long long n_dp, pwa_
     for (int q = 0; q < n_mj; ++q)
       if (p->mj[q].var == v) p->t_mj[t] = q;
   }
+  p->t_cols.clear();
+  p->t_col_beg.assign(1, 0);
+  for (int t = 0; t < p->n_train; ++t) {
+    for (int k = 0; k < p->ncol; ++k) {
+      bool in_col = p->t_mj[t] >= 0;
+      for (int f = 0; f < p->nfac; ++f)
+        in_col |= p->t_coup[t] >= 0 && p->col_fac[k * p->nfac + f] == p->t_coup[t];
+      if (in_col) p->t_cols.push_back(k);
+    }
+    p->t_col_beg.push_back((int)p->t_cols.size());
+  }
   p->key_var.clear();
   auto add_key = [&](int v) {
     if (v < 0) return;
@@ -588,7 +599,8 @@ void jacobian(pwa_hostprog* p, const double* vars, const std::vector<cd>& z,
       }
       const cd dzp = dz_at(ph_p, z[j]);
       const cd dzm = (role >= 2 ? -1.0 : 1.0) * dz_at(ph_m, p->zm[j]);
-      for (int k = 0; k < K; ++k) Jt[k] = prod_rule(k, j, z, dzp);
+      for (int c = p->t_col_beg[t]; c < p->t_col_beg[t + 1]; ++c)
+        Jt[p->t_cols[c]] = prod_rule(p->t_cols[c], j, z, dzp);
       if (Jmt)
         for (int c = 0; c < NC; ++c) Jmt[c] = prod_rule(p->cp_col[c], j, p->zm, dzm);
     }
@@ -619,7 +631,10 @@ void grad_from_sums(const pwa_hostprog* p, const cd* J, const cd* Jm, const doub
   for (int t = 0; t < p->n_train; ++t) {
     const cd* Jt = J + (long long)t * K;
     double acc = 0.0;
-    for (int k = 0; k < K; ++k) acc += Jt[k].real() * s[1 + 2 * k] - Jt[k].imag() * s[2 + 2 * k];
+    for (int c = p->t_col_beg[t]; c < p->t_col_beg[t + 1]; ++c) {
+      const int k = p->t_cols[c];
+      acc += Jt[k].real() * s[1 + 2 * k] - Jt[k].imag() * s[2 + 2 * k];
+    }
     if (Jm && p->cp_off >= 0) {
       // charge -1 column sums of the CP columns
       const cd* Jmt = Jm + (long long)t * NC;
@@ -627,7 +642,8 @@ void grad_from_sums(const pwa_hostprog* p, const cd* J, const cd* Jm, const doub
       for (int c = 0; c < NC; ++c) acc += Jmt[c].real() * sm[2 * c] - Jmt[c].imag() * sm[2 * c + 1];
     }
     acc *= 2.0;
-    for (int q = 0; q < NS; ++q) acc += D[(long long)t * NS + q] * s[1 + 2 * K + q];
+    if (p->t_sel[t] >= 0 || p->t_pol[t] >= 0)
+      for (int q = 0; q < NS; ++q) acc += D[(long long)t * NS + q] * s[1 + 2 * K + q];
     g[t] = acc;
   }
 }

@@ -79,6 +79,9 @@ struct pwa_hostprog {
   // 2 deltar, 3 deltai), shape selector slot or -1, barrier-row entry of mj
   // or -1, polarisation entry or -1
   std::vector<int> t_coup, t_comp, t_sel, t_mj, t_pol;
+  // columns that depend on each trainable variable: t_cols[t_col_beg[t] ..
+  // t_col_beg[t + 1]); the other Jacobian entries are zero
+  std::vector<int> t_cols, t_col_beg;
   // couplings and CP columns' couplings of the last consts() call, charge -1
   std::vector<std::complex<double>> zm;
   std::vector<double> ckm;

@@ -680,8 +680,8 @@ void split_tiles(long long td, long long tm, long long most, int* blocks, int* d
   *blocks = (int)(*data + (tm + r - 1) / r);
 }
 
-// Plain FP64 sums without the lineshape sums (pwa_eval_cols).
-int eval_cols(pwa_plan* h, const double* consts, cudaStream_t s, double* out) {
+// Launch of the plain FP64 sums without the lineshape sums (pwa_eval_cols).
+int eval_cols_enqueue(pwa_plan* h, const double* consts, cudaStream_t s) {
   if (!h->w) return set_err(h, PWA_ERR_STATE, "no events uploaded");
   if (h->ec_blocks == 0) {
     CU(cudaFuncSetAttribute((const void*)h->k.eval_cols,
@@ -708,7 +708,7 @@ int eval_cols(pwa_plan* h, const double* consts, cudaStream_t s, double* out) {
                                    args, (size_t)h->ec_smem, s);
   if (e != cudaSuccess)
     return set_err(h, PWA_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e));
-  return wait_mapped_sums(h, s, out);
+  return PWA_OK;
 }
 
 // Whether no trainable variable takes a derivative through the kernels'
@@ -2223,19 +2223,27 @@ int pwa_hostprog_jacobian(pwa_hostprog* p, const double* vars, double* J, double
 }
 
 namespace {
+// Jacobian of one parameter vector (pwa_host::jacobian)
+struct HpJacobian {
+  std::vector<std::complex<double>> J, Jm;
+  std::vector<double> D;
+  HpJacobian(pwa_hostprog* p, const double* vars, const std::vector<std::complex<double>>& z,
+             const std::vector<double>& ck)
+      : J((size_t)p->n_train * p->ncol),
+        Jm((size_t)p->n_train * p->cp_col.size() + 1),
+        D((size_t)p->n_train * p->nshape + 1) {
+    pwa_host::jacobian(p, vars, z, ck, J.data(), Jm.data(), D.data());
+  }
+};
 // piece vector [S_d, S_m*share, sw, g_d, g_m*share] from the data and MC sums
-void pieces_from_hp_sums(pwa_hostprog* p, const double* vars, const std::vector<std::complex<double>>& z,
-                         const std::vector<double>& ck, const double* sd, const double* sm,
-                         double sw, double mc_share, double* out) {
+void pieces_from_hp_sums(const pwa_hostprog* p, const HpJacobian& j, const double* sd,
+                         const double* sm, double sw, double mc_share, double* out) {
   const int P = p->n_train;
-  std::vector<std::complex<double>> J((size_t)P * p->ncol), Jm((size_t)P * p->cp_col.size() + 1);
-  std::vector<double> D((size_t)P * p->nshape + 1);
-  pwa_host::jacobian(p, vars, z, ck, J.data(), Jm.data(), D.data());
   out[0] = sd[0];
   out[1] = sm[0] * mc_share;
   out[2] = sw;
-  pwa_host::grad_from_sums(p, J.data(), Jm.data(), D.data(), sd, out + 3);
-  pwa_host::grad_from_sums(p, J.data(), Jm.data(), D.data(), sm, out + 3 + P);
+  pwa_host::grad_from_sums(p, j.J.data(), j.Jm.data(), j.D.data(), sd, out + 3);
+  pwa_host::grad_from_sums(p, j.J.data(), j.Jm.data(), j.D.data(), sm, out + 3 + P);
   for (int t = 0; t < P; ++t) out[3 + P + t] *= mc_share;
 }
 }  // namespace
@@ -2246,7 +2254,7 @@ int pwa_hostprog_pieces(pwa_hostprog* p, const double* vars, const double* sd, c
   std::vector<double> C(p->nconst), ck;
   std::vector<std::complex<double>> z;
   pwa_host::consts(p, vars, C.data(), &z, &ck);
-  pieces_from_hp_sums(p, vars, z, ck, sd, sm, sw, mc_share, out);
+  pieces_from_hp_sums(p, HpJacobian(p, vars, z, ck), sd, sm, sw, mc_share, out);
   return PWA_OK;
 }
 
@@ -2289,20 +2297,24 @@ int pwa_pieces_vars(pwa_plan* h, const double* vars, int form, double sw, double
     if (pwa_host::column_rho(p, C.data(), rho.data()) &&
         pwa_host::column_rho(p, h->sc_consts.data(), rho0.data())) {
       for (int k = 0; k < h->ncol; ++k) rho[k] /= rho0[k];
-      rc = pwa_eval_shapecache(h, C.data(), rho.data(), stream, sums.data());
+      rc = pwa_eval_shapecache_enqueue(h, C.data(), rho.data(), stream);
     } else {
       // a normalisation is not positive here: the columns do not factorise,
       // so this point recomputes them (FP32 amplitudes)
-      rc = pwa_eval(h, C.data(), PWA_MIXED_F32, 1, stream, sums.data());
+      rc = pwa_eval_enqueue(h, C.data(), PWA_MIXED_F32, 1, stream);
     }
   } else if (form == PWA_FORM_PLAIN_F64 && h->ec_smem > 0 && no_shape_sums(*p)) {
-    rc = eval_cols(h, C.data(), (cudaStream_t)stream, sums.data());
+    rc = eval_cols_enqueue(h, C.data(), (cudaStream_t)stream);
   } else {
-    rc = pwa_eval(h, C.data(), form == PWA_FORM_PLAIN_F64 ? PWA_PLAIN_F64 : PWA_MIXED_F32, 1,
-                  stream, sums.data());
+    rc = pwa_eval_enqueue(h, C.data(), form == PWA_FORM_PLAIN_F64 ? PWA_PLAIN_F64 : PWA_MIXED_F32,
+                          1, stream);
   }
   if (rc) return rc;
-  pieces_from_hp_sums(p, vars, z, ck, sums.data(), sums.data() + h->nacc, sw, mc_share, out);
+  // the Jacobian while the device forms the sums
+  const HpJacobian jac(p, vars, z, ck);
+  rc = wait_mapped_sums(h, (cudaStream_t)stream, sums.data());
+  if (rc) return rc;
+  pieces_from_hp_sums(p, jac, sums.data(), sums.data() + h->nacc, sw, mc_share, out);
   return PWA_OK;
 }
 

@@ -20,6 +20,7 @@ derivative of the column's log barrier factors through q0 (nominal masses).
 import cmath
 import ctypes
 import os
+import struct
 
 import numpy as np
 
@@ -232,6 +233,12 @@ class HostProgram:
             self.close()
         except Exception:
             pass
+
+
+def _fill(buf, values):
+    """buf[:] = values for a sequence of Python floats (134 of them: 2 us
+    instead of 5 through an array)."""
+    struct.pack_into(f"{len(buf)}d", buf, 0, *values)
 
 
 def _dptr(a):
@@ -1263,7 +1270,7 @@ class Engine:
         if self.dist_reduce is not None:
             vec = self.dist_reduce(self.pieces_vars(var_values, form, stream=stream))
             return combine_pieces(vec, self._hp_train)
-        self._hp_vbuf[:] = var_values
+        _fill(self._hp_vbuf, var_values)
         pv, pg, pn = self._hp_ptrs
         self._check(load_library().pwa_nll_grad_vars(self.h, pv, int(form), self._sw,
                                                      stream or 0, pn, pg), "pwa_nll_grad_vars")
@@ -1291,7 +1298,7 @@ class Engine:
         if self.dist_reduce is not None:
             vec = self.dist_reduce(self.pieces_cached(var_values, stream=stream))
             return combine_pieces(vec, self._n_train)
-        self._vbuf[:] = var_values
+        _fill(self._vbuf, var_values)
         self._check(load_library().pwa_nll_grad_cached(self.h, self._vbuf_p, self._sw,
                                                        stream or 0, self._nbuf_p, self._gbuf_p),
                     "pwa_nll_grad_cached")
