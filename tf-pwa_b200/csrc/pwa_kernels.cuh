@@ -381,16 +381,21 @@ extern "C" __global__ void __launch_bounds__(PWA_TPB)
   }
 }
 
-// Column-wise deterministic sum of nrows rows of width ncols.
+// Column-wise deterministic sum of nrows rows of width ncols, into out, or
+// (seq != 0) as result entries into mapped host memory.
 extern "C" __global__ void pwa_sum_rows(const double* __restrict__ in, int nrows, int ncols,
-                                        double* __restrict__ out) {
+                                        double* __restrict__ out, unsigned int seq) {
   const int lane = threadIdx.x & 31;
   const int warps = blockDim.x >> 5;
   for (int j = (int)(blockIdx.x * warps + (threadIdx.x >> 5)); j < ncols; j += gridDim.x * warps) {
     double s = 0.0;
+#pragma unroll 4
     for (int r = lane; r < nrows; r += 32) s += in[(long long)r * ncols + j];
     s = warp_sum(s);
-    if (lane == 0) out[j] = s;
+    if (lane == 0) {
+      if (seq) ll_store(out, j, s, seq);
+      else out[j] = s;
+    }
   }
 }
 

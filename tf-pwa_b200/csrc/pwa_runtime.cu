@@ -132,7 +132,6 @@ struct pwa_plan {
   // plain FP64 evaluation from the columns (pwa_eval_cols): shared memory of
   // a block (0: the model keeps pwa_eval_f64) and its grid (0: not set up)
   int ec_smem = 0, ec_blocks = 0, ec_blocks_data = 0;
-  double* d_hsum = nullptr;
   // parameter layout for the C-side chain rule
   int n_vars = 0, n_coup = 0, nfac = 0, n_train = 0;
   std::vector<int> coup_r, coup_i, coup_polar, col_fac, train_idx;
@@ -517,7 +516,6 @@ int pwa_plan_destroy(pwa_plan* h) {
   if (h->d_multi) cudaFree(h->d_multi);
   if (h->h_mbig) cudaFreeHost(h->h_mbig);
   if (h->d_pts) cudaFree(h->d_pts);
-  if (h->d_hsum) cudaFree(h->d_hsum);
   if (h->scache) cudaFree(h->scache);
   if (h->h_pin) cudaFreeHost(h->h_pin);
   if (h->lib) cudaLibraryUnload(h->lib);
@@ -652,6 +650,42 @@ bool wait_result(pwa_plan* h, const double* mapped, int n, cudaStream_t s, doubl
     std::memcpy(&h->sums[j], &b, sizeof(double));
   }
   return true;
+}
+
+// A pinned mapped area of `bytes` (host and device address) for the arguments
+// or results of one call: the plan's own block, or one grown to fit.
+int pinned_io(pwa_plan* h, size_t bytes, char** hp, char** dp) {
+  *hp = h->h_pin + h->pin_batch;
+  *dp = h->d_pin + h->pin_batch;
+  if (bytes <= h->pin_batch_cap) return PWA_OK;
+  if (bytes > h->mbig_cap) {
+    if (h->h_mbig) cudaFreeHost(h->h_mbig);
+    h->h_mbig = h->d_mbig = nullptr;
+    h->mbig_cap = 0;
+    if (cudaHostAlloc(&h->h_mbig, 2 * bytes, cudaHostAllocMapped) != cudaSuccess)
+      return set_err(h, PWA_ERR_OOM, "allocation of pinned memory failed");
+    CU(cudaHostGetDevicePointer((void**)&h->d_mbig, h->h_mbig, 0));
+    h->mbig_cap = 2 * bytes;
+  }
+  *hp = h->h_mbig;
+  *dp = h->d_mbig;
+  return PWA_OK;
+}
+
+// Column sums of `nrows` rows of `ncols` in h->partials (pwa_sum_rows), through
+// mapped memory into h->sums: no copy and no stream synchronisation.
+int sum_partial_rows(pwa_plan* h, int nrows, int ncols, cudaStream_t s) {
+  char *hp = nullptr, *dp = nullptr;
+  int rc = pinned_io(h, 16 * (size_t)ncols, &hp, &dp);
+  if (rc) return rc;
+  std::memset(hp, 0, 16 * (size_t)ncols);  // other calls' contents: no number of this one
+  unsigned int seq = next_seq(h);
+  void* args[] = {&h->partials, &nrows, &ncols, &dp, &seq};
+  rc = launch(h, h->k.sum_rows, dim3((unsigned)((ncols + 7) / 8)), dim3(256), args, s);
+  if (rc) return rc;
+  if (!wait_result(h, (const double*)hp, ncols, s, 1.0))
+    return set_err(h, PWA_ERR_CUDA, "sums did not arrive (stale result)");
+  return PWA_OK;
 }
 
 // The data and MC sums of the last plain, FP32 or floating-shape evaluation.
@@ -927,7 +961,8 @@ int gram_tc_chunk(pwa_plan* h, double* F, double* wptr, long long cnt, double* g
   if (e != cudaSuccess)
     return set_err(h, PWA_ERR_CUDA, std::string("gram kernel launch: ") + cudaGetErrorString(e));
   int nrows = gb, ncols = KC * KC;
-  void* a3[] = {&gpart, &nrows, &ncols, &gsum};
+  unsigned int plain = 0;
+  void* a3[] = {&gpart, &nrows, &ncols, &gsum, &plain};
   rc = launch(h, h->k.sum_rows, dim3(16), dim3(256), a3, s);
   if (rc) return rc;
   std::vector<double> G((size_t)KC * KC);
@@ -978,7 +1013,7 @@ int gram_fused(pwa_plan* h, const std::vector<double>& cbuf, size_t smem, int ti
   if (per_sm < 1) per_sm = 1;
   const long long want = (long long)per_sm * h->sms, need = (h->n_mc + h->tpb - 1) / h->tpb;
   int nrows = (int)(want < need ? want : need), ncols = tiles * 64;
-  int rc = ensure_partials(h, ((long long)nrows + 1) * ncols);
+  int rc = ensure_partials(h, (long long)nrows * ncols);
   if (rc) return rc;
   long long beg = h->n_data, end = h->n_data + h->n_mc, ld = h->ld;
   void* a1[] = {(void*)cbuf.data(), &h->xa, &h->xm, &h->w, &beg, &end, &ld, &h->partials};
@@ -986,18 +1021,13 @@ int gram_fused(pwa_plan* h, const std::vector<double>& cbuf, size_t smem, int ti
                                    smem, s);
   if (e != cudaSuccess)
     return set_err(h, PWA_ERR_CUDA, std::string("gram kernel launch: ") + cudaGetErrorString(e));
-  double* gsum = h->partials + (long long)nrows * ncols;
-  void* a2[] = {&h->partials, &nrows, &ncols, &gsum};
-  rc = launch(h, h->k.sum_rows, dim3((ncols + 7) / 8), dim3(256), a2, s);
+  rc = sum_partial_rows(h, nrows, ncols, s);
   if (rc) return rc;
-  std::vector<double> t((size_t)ncols);
-  CU(cudaMemcpyAsync(t.data(), gsum, sizeof(double) * ncols, cudaMemcpyDeviceToHost, s));
-  CU(cudaStreamSynchronize(s));
   // real symmetric G from its lower tiles: lane l holds row l / 4, columns
   // 2 (l % 4), 2 (l % 4) + 1 of an 8 x 8 tile
   const int K = h->ncol, cp = (2 * K + 7) / 8 * 8;
   std::vector<double> G((size_t)cp * cp, 0.0);
-  const double* q = t.data();
+  const double* q = h->sums.data();
   for (int bi = 0; bi < cp / 8; ++bi)
     for (int bj = 0; bj <= bi; ++bj, q += 64)
       for (int l = 0; l < 32; ++l)
@@ -1081,7 +1111,8 @@ int pwa_build_gram(pwa_plan* h, const double* consts, void* stream, double* out)
     rc = launch(h, h->k.gram_f64, dim3(gb), dim3(h->tpb), a2, s);
     if (rc) break;
     int nrows = gb, ncols = (int)nkk;
-    void* a3[] = {&gpart, &nrows, &ncols, &gsum};
+    unsigned int plain = 0;
+    void* a3[] = {&gpart, &nrows, &ncols, &gsum, &plain};
     rc = launch(h, h->k.sum_rows, dim3(16), dim3(256), a3, s);
     if (rc) break;
     if (cudaMemcpyAsync(part.data(), gsum, sizeof(double) * nkk, cudaMemcpyDeviceToHost, s) !=
@@ -1738,20 +1769,9 @@ int pwa_pieces_multi(pwa_plan* h, int n_req, const long long* first_tile, const 
   // pinned arguments and mapped result
   const size_t meta_bytes = (words * 8 + 255) / 256 * 256;
   const size_t pin_bytes = meta_bytes + sizeof(double) * ((size_t)n_req * NA + 1);
-  char *h_io = h->h_pin + h->pin_batch, *d_io = h->d_pin + h->pin_batch;
-  if (pin_bytes > h->pin_batch_cap) {
-    if (pin_bytes > h->mbig_cap) {
-      if (h->h_mbig) cudaFreeHost(h->h_mbig);
-      h->h_mbig = h->d_mbig = nullptr;
-      h->mbig_cap = 0;
-      if (cudaHostAlloc(&h->h_mbig, 2 * pin_bytes, cudaHostAllocMapped) != cudaSuccess)
-        return set_err(h, PWA_ERR_OOM, "allocation of the batch arguments failed");
-      CU(cudaHostGetDevicePointer((void**)&h->d_mbig, h->h_mbig, 0));
-      h->mbig_cap = 2 * pin_bytes;
-    }
-    h_io = h->h_mbig;
-    d_io = h->d_mbig;
-  }
+  char *h_io = nullptr, *d_io = nullptr;
+  int rc = pinned_io(h, pin_bytes, &h_io, &d_io);
+  if (rc) return rc;
   long long* cbeg = (long long*)h_io;
   long long *tbeg = cbeg + n_req + 1, *gbeg = tbeg + n_req + 1, *first = gbeg + n_req + 1,
             *cs = first + n_req;
@@ -1815,7 +1835,7 @@ int pwa_pieces_multi(pwa_plan* h, int n_req, const long long* first_tile, const 
   h_res[(size_t)n_req * NA] = -1.0;  // the mark's place follows the request count
   void* a1[] = {&d_meta, &n_req, &n_chunks, &n_work, &n_groups, &h->pool_f, &h->pool_w,
                 &d_rows, &d_count, &d_res, &seq};
-  int rc = launch(h, h->k.eval_multi, dim3((int)nb), dim3(h->tpb), a1, s);
+  rc = launch(h, h->k.eval_multi, dim3((int)nb), dim3(h->tpb), a1, s);
   if (rc) return rc;
   // the Gram part and the Jacobians while the device forms the data sums
   std::vector<cplx> J(h->jac.size() * (size_t)n_req);
@@ -1952,8 +1972,6 @@ int hess_sums(pwa_plan* h, const double* ck, cudaStream_t s, double* out) {
                                                      smem));
     if (per < 1) return set_err(h, PWA_ERR_STATE, "exact Hessian kernel does not fit an SM");
     const long long want = (long long)per * h->sms;
-    if (!h->d_hsum && cudaMalloc(&h->d_hsum, sizeof(double) * NA) != cudaSuccess)
-      return set_err(h, PWA_ERR_OOM, "cudaMalloc of the Hessian sums failed");
     h->hess_smem = smem;
     h->hess_blocks = (int)(want < h->ntiles ? want : h->ntiles);
   }
@@ -1966,12 +1984,9 @@ int hess_sums(pwa_plan* h, const double* ck, cudaStream_t s, double* out) {
                                    dim3(h->tpb), args, h->hess_smem, s);
   if (e != cudaSuccess)
     return set_err(h, PWA_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e));
-  int nrows = h->hess_blocks, ncols = (int)NA;
-  void* a2[] = {&h->partials, &nrows, &ncols, &h->d_hsum};
-  rc = launch(h, h->k.sum_rows, dim3((unsigned)((NA + 7) / 8)), dim3(256), a2, s);
+  rc = sum_partial_rows(h, h->hess_blocks, (int)NA, s);
   if (rc) return rc;
-  CU(cudaMemcpyAsync(out, h->d_hsum, sizeof(double) * NA, cudaMemcpyDeviceToHost, s));
-  CU(cudaStreamSynchronize(s));
+  std::copy(h->sums.begin(), h->sums.end(), out);
   return PWA_OK;
 }
 
