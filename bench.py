@@ -62,14 +62,14 @@ NCU_TRAFFIC_PER_ROW = {"lc2pkpi": (290.436096e6 + 6.841088e6) / 1.1e6,
                        "b2dstkpi": (248.044032e6 + 3.609856e6) / 1e6}
 # the same for the floating-shape evaluation kernel, per event (data + MC):
 # D -> K pi pi, 80.04 + 2.29 MB for 2e6 events
-# (Lambda_c: 151.30 + 5.62 MB for the 5.25e5 events of a quarter-size
+# (Lambda_c: 151.28 + 3.08 MB for the 5.25e5 events of a quarter-size
 # capture, inputs larger than L2; traffic grows with the events)
 NCU_SC_TRAFFIC_PER_EVENT = {"d2kpipi_float": (80.041728e6 + 2.286848e6) / 2e6,
-                            "lc2pkpi_float": (151.29728e6 + 5.616384e6) / 5.25e5}
+                            "lc2pkpi_float": (151.282432e6 + 3.076352e6) / 5.25e5}
 # its FP64 operations per event (2 DFMA + DMUL + DADD executed, ncu; 5e5 and
 # 5.25e5 events)
-NCU_SC_F64_FLOPS_PER_EVENT = {"d2kpipi_float": (2 * 54011168 + 33358304 + 17445502) / 5e5,
-                              "lc2pkpi_float": (2 * 222667712 + 81638424 + 38105098) / 5.25e5}
+NCU_SC_F64_FLOPS_PER_EVENT = {"d2kpipi_float": (2 * 38159312 + 29462416 + 16747908) / 5e5,
+                              "lc2pkpi_float": (2 * 220131984 + 70388192 + 44628976) / 5.25e5}
 
 
 def _select(name):
@@ -596,6 +596,8 @@ def measure_cached(name, args, rank, world, dist, timed, log, n_sig, n_bg, n_mc,
                          "launch_us": 1e6 * t_floor / k_kernel,
                          "kernel_over_floor": t_kernel / t_floor},
                      "plain_f64_kernel": {
+                         "kernel": "pwa_eval_f64 (with the lineshape sums; the plain_f64 "
+                                   "evaluations above, without them, run pwa_eval_cols)",
                          "bound": "fp64", "achieved": ach_p, "peak": peaks["f64_tflops"],
                          "unit": "TFLOP/s", "frac": ach_p / peaks["f64_tflops"],
                          "peak_kind": "measured here (pwa_fma_peak, FP64 FMA chains)",
@@ -714,7 +716,7 @@ def measure_floating(name, args, rank, world, dist, timed, log, n_sig, n_mc, n_b
     peaks = {"f64_tflops": fcn.eng.fma_peak(PLAIN_F64) / 1e12,
              "f32_tflops": fcn.eng.fma_peak(MIXED_F32) / 1e12}
     roof_r = _mixed_pipe_roofline(name, n_all, t_k / args.steps, peaks)
-    roof_r.update({"kernel": "pwa_eval_f32 + pwa_reduce (data + MC, FP32 amplitudes)",
+    roof_r.update({"kernel": "pwa_eval_f32 with its own reduction (data + MC, FP32 amplitudes)",
                    "hbm": {"achieved": ach, "peak": hbm, "unit": "GB/s", "frac": ach / hbm,
                            "peak_kind": peak_kind, "algorithmic_bytes_per_launch": bytes_f32}})
     fl_p = NCU_F64_FLOPS_PER_EVENT[name]
@@ -743,6 +745,7 @@ def measure_floating(name, args, rank, world, dist, timed, log, n_sig, n_mc, n_b
                   "FP64 masses, lineshapes recomputed)",
         "algorithmic_bytes_per_launch": bytes_sc, "launch_us": 1e6 * t_ks / args.steps,
         "plain_f64_kernel": {
+            "kernel": "pwa_eval_f64",
             "bound": "fp64", "achieved": ach_p, "peak": peaks["f64_tflops"],
             "unit": "TFLOP/s", "frac": ach_p / peaks["f64_tflops"], "flops_per_event": fl_p,
             "flops_source": "ncu: 2 DFMA + DADD + DMUL executed per event (forward and "

@@ -208,11 +208,13 @@ int pwa_read_dat(const char* path, double* out, long long cap, long long* n_valu
 int pwa_build_gram(pwa_plan* h, const double* consts, void* stream, double* out);
 
 /* How pwa_build_gram contracts the columns (tf_pwa/model/opt_int.py:128-296
- * builds the same matrix with a TF einsum): 0 = FP64 on the CUDA cores,
+ * builds the same matrix with a TF einsum): 0 = FP64 matrix instructions in
+ * the kernel that forms the columns (models whose tile does not fit in
+ * shared memory: columns to memory, FP64 on the CUDA cores),
  * 1 = tensor cores (tcgen05 int8 MMAs on seven exact slices of every value,
  * exact int32 accumulation, FP64 recombination; models with at most 32
  * columns, others use 0), -1 = automatic (0: at the shipped models' column
- * counts the slicing costs more than the FP64 products it replaces).  The
+ * counts the slicing alone costs more than the whole of 0).  The
  * error flag of the tensor-core kernel turns into PWA_ERR_CUDA. */
 int pwa_set_gram_method(pwa_plan* h, int method);
 

@@ -432,7 +432,7 @@ __device__ __forceinline__ void stage_sp(const Consts& C, double* s_sp) {
 // (columns to memory, 480 B per four-body event, then one thread per (k, l)
 // reading two operands per product from shared memory, and a 256 MB buffer
 // allocated and freed per call): a whole fit set-up, column cache of 3e5 and
-// Gram of 1.2e6 four-body events, took 5.1 ms and takes 0.60 ms.  Models
+// Gram of 1.2e6 four-body events, took 5.1 ms and takes 0.58 ms.  Models
 // whose tile exceeds GM_MAX_BYTES (many helicities x columns: two blocks
 // would not fit on an SM) keep that form.
 #define GM_CP ((2 * PWA_NCOL + 7) / 8 * 8)
@@ -1222,8 +1222,8 @@ extern "C" __global__ void __launch_bounds__(PWA_TPB, PWA_SC_MINB)
 // halves for data and MC blocks, result in mapped memory, one launch.
 // Bound: the FP64 pipe and its latency at three blocks per SM (shared
 // memory).  Measured against pwa_eval_f64 and its reduce launch, whole
-// evaluations: four-body 1e6 events 237 vs 1098 us, Lambda_c 2.1e6 379 vs
-// 655 us, D -> K pi pi 1.1e5 23 vs 29 us.
+// evaluations: four-body 1e6 events 217 vs 1098 us, Lambda_c 2.1e6 379 vs
+// 655 us, D -> K pi pi 1.1e5 20 vs 29 us.
 // Models with a density matrix, per-charge totals or more pairs than fit
 // (EC_MAX_BYTES) keep pwa_eval_f64, as do evaluations with free masses or
 // widths, which need the lineshape sums.
