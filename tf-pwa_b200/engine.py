@@ -1364,7 +1364,9 @@ class Engine:
         import torch
 
         n = p4.shape[0]
-        p4 = p4.to(torch.float64)
+        # read through its pointer: a lazily negated view (the imaginary part
+        # of a conjugated tensor) has its values formed first
+        p4 = p4.to(torch.float64).resolve_neg()
         ci = self.plan.charge_index
         ch = None
         if self.plan.use_charge and charge is not None:
