@@ -236,9 +236,13 @@ class HostProgram:
 
 
 def _fill(buf, values):
-    """buf[:] = values for a sequence of Python floats (134 of them: 2 us
-    instead of 5 through an array)."""
-    struct.pack_into(f"{len(buf)}d", buf, 0, *values)
+    """buf[:] = values; a sequence of len(buf) numbers is packed directly (134
+    Python floats: 2 us instead of 5 through an array).  What cannot be packed
+    takes the assignment, which broadcasts, converts or raises."""
+    try:
+        struct.pack_into(f"{len(buf)}d", buf, 0, *values)
+    except (struct.error, TypeError):
+        buf[:] = values
 
 
 def _dptr(a):
