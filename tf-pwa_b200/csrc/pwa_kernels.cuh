@@ -2733,8 +2733,10 @@ extern "C" __global__ void __launch_bounds__(PWA_TPB, PWA_MULTI_MINB)
     }
     t1 = t + cs < te ? t + cs : te;
   }
-  __threadfence();
+  // every row of the block written, then a fence of the counting lanes: their
+  // counts carry the whole block's rows
   __syncthreads();
+  __threadfence();
   // count the block's chunks in: lane l of warp v takes group v + NW l of the
   // groups that [ca, cb) touches, then 32 NW further
   double* grow = rows + n_chunks * NW * NA;
@@ -2753,12 +2755,16 @@ extern "C" __global__ void __launch_bounds__(PWA_TPB, PWA_MULTI_MINB)
       full = atomicAdd(count + g, mine) + mine == (unsigned)(b1 - b0);
     }
     unsigned todo = __ballot_sync(0xffffffffu, full);
+    // the counting lane's fence, then a warp barrier: only with both are the
+    // other lanes' reads of the rows behind its count (a vote or a shuffle
+    // orders no memory)
+    __threadfence();
+    __syncwarp();
     while (todo) {
       const int src = __ffs(todo) - 1;
       todo &= todo - 1;
       const long long gg = gw + NW * src;
       const int qq = __shfl_sync(0xffffffffu, q, src);
-      __threadfence();
       const long long g0 = __ldg(m.gbeg + qq), ng = __ldg(m.gbeg + qq + 1) - g0;
       const long long b0 = __ldg(m.cbeg + qq) + (gg - g0) * PWA_MGROUP;
       const long long qe = __ldg(m.cbeg + qq + 1);
@@ -2769,9 +2775,10 @@ extern "C" __global__ void __launch_bounds__(PWA_TPB, PWA_MULTI_MINB)
         count[gg] = 0u;
         __threadfence();
         last = atomicAdd(count + n_groups + qq, 1u) == (unsigned)ng - 1;
+        __threadfence();
       }
+      __syncwarp();  // the group rows' reads behind lane 0's count
       if (!__shfl_sync(0xffffffffu, last, 0)) continue;
-      __threadfence();
       multi_sum_rows(grow + g0 * NA, ng, out + (long long)qq * NA, lane);
       if (lane == 0) {
         count[n_groups + qq] = 0u;
