@@ -105,7 +105,11 @@ int pwa_eval(pwa_plan* h, const double* consts, int precision, int mc, void* str
 
 /* The device work of pwa_eval (fused kernel + fixed-order reduction) only,
  * enqueued on `stream` without waiting; the sums stay on the device.  For
- * timing the kernels and for capture into larger asynchronous pipelines. */
+ * timing the kernels and for capture into larger asynchronous pipelines.  A
+ * captured launch keeps the plan's block rows: evaluations and
+ * pwa_build_gram on the same events leave them in place; capture after the
+ * column caches and the first Hessian or multi-point call, which may enlarge
+ * them, and again after an upload. */
 int pwa_eval_enqueue(pwa_plan* h, const double* consts, int precision, int mc, void* stream);
 
 /* Per-event sum |A|^2 of events [beg, end) of the uploaded set into

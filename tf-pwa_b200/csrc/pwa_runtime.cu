@@ -130,7 +130,8 @@ struct pwa_plan {
   int sc_smem = 0;    // dynamic shared memory of pwa_eval_shapecache
   bool shape_cache_ok = false;  // the model's columns factorise (PWA_SHAPE_CACHE_OK 1)
   // plain FP64 evaluation from the columns (pwa_eval_cols): shared memory of
-  // a block (0: the model keeps pwa_eval_f64) and its grid (0: not set up)
+  // a block (0: the model keeps pwa_eval_f64) and its grid (0: no
+  // events uploaded)
   int ec_smem = 0, ec_blocks = 0, ec_blocks_data = 0;
   // parameter layout for the C-side chain rule
   int n_vars = 0, n_coup = 0, nfac = 0, n_train = 0;
@@ -186,13 +187,15 @@ constexpr int kTicketWords = 2 + 4096;
 // must be a multiple of this
 constexpr int kTmaGroups = 2;
 
+// Block rows of at least n doubles.  The old ones go only when the new ones
+// are there: a growth that fails leaves the plan's other calls as they were.
 int ensure_partials(pwa_plan* h, long long n) {
   if (n <= h->partials_cap) return PWA_OK;
-  if (h->partials) cudaFree(h->partials);
-  h->partials = nullptr;
-  h->partials_cap = 0;
-  if (cudaMalloc(&h->partials, sizeof(double) * n) != cudaSuccess)
+  double* p = nullptr;
+  if (cudaMalloc(&p, sizeof(double) * n) != cudaSuccess)
     return set_err(h, PWA_ERR_OOM, "cudaMalloc partials failed");
+  if (h->partials) cudaFree(h->partials);
+  h->partials = p;
   h->partials_cap = n;
   return PWA_OK;
 }
@@ -523,6 +526,77 @@ int pwa_plan_destroy(pwa_plan* h) {
   return PWA_OK;
 }
 
+namespace {
+// Blocks for td data and tm MC tiles on at most `most` blocks: the fewest
+// tiles r per block for which both sets' blocks fit, so that no block takes
+// one tile more than the others (a split in proportion to the events rounds
+// one set's share up and leaves its blocks a whole tile behind).
+void split_tiles(long long td, long long tm, long long most, int* blocks, int* data) {
+  long long r = (td + tm + most - 1) / most;
+  if (r < 1) r = 1;
+  while ((td + r - 1) / r + (tm + r - 1) / r > most) ++r;
+  *data = (int)((td + r - 1) / r);
+  *blocks = (int)(*data + (tm + r - 1) / r);
+}
+
+// Shared memory of one block of pwa_gram_fused and its count of 8 x 8 tiles
+// (GM_* of the device header); 0 bytes where the kernel is compiled empty.
+size_t gram_fused_bytes(const pwa_plan* h, int* tiles) {
+  const int cp = (2 * h->ncol + 7) / 8 * 8, nt = cp / 8;
+  *tiles = nt * (nt + 1) / 2;
+  const size_t bytes = (size_t)h->nout * h->tpb * (cp + 4) * sizeof(double);
+  return bytes <= 104 * 1024 && *tiles <= 12 * (h->tpb / 32) ? bytes : 0;
+}
+
+// Blocks of pwa_gram_fused over the MC events, and its shared memory allowed.
+int gram_fused_grid(pwa_plan* h, size_t smem, int* nrows) {
+  CU(cudaFuncSetAttribute((const void*)h->k.gram_fused,
+                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  int per_sm = 0;
+  CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)h->k.gram_fused, h->tpb,
+                                                   smem));
+  if (per_sm < 1) per_sm = 1;
+  const long long want = (long long)per_sm * h->sms, need = (h->n_mc + h->tpb - 1) / h->tpb;
+  *nrows = (int)(want < need ? want : need);
+  return PWA_OK;
+}
+
+// The grid of pwa_eval_cols, and the block rows of every kernel that
+// evaluates the uploaded events as they are: evaluations and the Gram matrix
+// never move them afterwards, so launches captured with pwa_eval_enqueue stay
+// valid beside them.
+int reserve_block_rows(pwa_plan* h) {
+  long long rows = h->nblocks > h->nblocks32 ? h->nblocks : h->nblocks32;
+  int nb = 0, bd = 0;
+  if (h->ec_smem > 0) {
+    CU(cudaFuncSetAttribute((const void*)h->k.eval_cols,
+                            cudaFuncAttributeMaxDynamicSharedMemorySize, h->ec_smem));
+    int per_sm = 0;
+    CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)h->k.eval_cols, h->tpb,
+                                                     h->ec_smem));
+    if (per_sm < 1) per_sm = 1;
+    const long long t = h->tpb;
+    split_tiles((h->n_data + t - 1) / t, (h->n_mc + t - 1) / t, (long long)per_sm * h->sms, &nb,
+                &bd);
+    if (nb > rows) rows = nb;
+  }
+  // block rows of 2 nacc and the group rows of the in-kernel reduction
+  long long need = (rows + (rows + 15) / 16) * 2 * h->nacc;
+  int tiles = 0, nrows = 0;
+  const size_t smem = gram_fused_bytes(h, &tiles);
+  if (smem && h->n_mc > 0) {
+    const int rc = gram_fused_grid(h, smem, &nrows);
+    if (rc) return rc;
+    if ((long long)nrows * tiles * 64 > need) need = (long long)nrows * tiles * 64;
+  }
+  const int rc = ensure_partials(h, need);
+  if (rc) return rc;
+  h->ec_blocks = nb;
+  h->ec_blocks_data = bd;
+  return PWA_OK;
+}
+}  // namespace
+
 int pwa_upload_events(pwa_plan* h, const double* xm, const double* xa, const double* w,
                       long long n_data, long long n_mc, int on_device, void* stream) {
   if (!h) return PWA_ERR_ARG;
@@ -587,9 +661,7 @@ int pwa_upload_events(pwa_plan* h, const double* xm, const double* xa, const dou
   };
   CU(grid(h->k.eval_f64, &h->nblocks, &h->blocks_data));
   CU(grid(h->k.eval_f32, &h->nblocks32, &h->blocks_data32));
-  const int nb_max = h->nblocks > h->nblocks32 ? h->nblocks : h->nblocks32;
-  // block rows of 2 nacc and the group rows of the in-kernel reduction
-  int rc = ensure_partials(h, (long long)(nb_max + (nb_max + 15) / 16) * 2 * h->nacc);
+  const int rc = reserve_block_rows(h);
   if (rc) return rc;
   CU(cudaStreamSynchronize(s));
   return PWA_OK;
@@ -702,37 +774,9 @@ int wait_mapped_sums(pwa_plan* h, cudaStream_t s, double* out) {
 }  // namespace
 
 namespace {
-// Blocks for td data and tm MC tiles on at most `most` blocks: the fewest
-// tiles r per block for which both sets' blocks fit, so that no block takes
-// one tile more than the others (a split in proportion to the events rounds
-// one set's share up and leaves its blocks a whole tile behind).
-void split_tiles(long long td, long long tm, long long most, int* blocks, int* data) {
-  long long r = (td + tm + most - 1) / most;
-  if (r < 1) r = 1;
-  while ((td + r - 1) / r + (tm + r - 1) / r > most) ++r;
-  *data = (int)((td + r - 1) / r);
-  *blocks = (int)(*data + (tm + r - 1) / r);
-}
-
 // Launch of the plain FP64 sums without the lineshape sums (pwa_eval_cols).
 int eval_cols_enqueue(pwa_plan* h, const double* consts, cudaStream_t s) {
-  if (!h->w) return set_err(h, PWA_ERR_STATE, "no events uploaded");
-  if (h->ec_blocks == 0) {
-    CU(cudaFuncSetAttribute((const void*)h->k.eval_cols,
-                            cudaFuncAttributeMaxDynamicSharedMemorySize, h->ec_smem));
-    int per_sm = 0;
-    CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)h->k.eval_cols, h->tpb,
-                                                     h->ec_smem));
-    if (per_sm < 1) per_sm = 1;
-    const long long t = h->tpb;
-    int nb = 0, bd = 0;
-    split_tiles((h->n_data + t - 1) / t, (h->n_mc + t - 1) / t, (long long)per_sm * h->sms, &nb,
-                &bd);
-    const int rc = ensure_partials(h, (long long)(nb + (nb + 15) / 16) * 2 * h->nacc);
-    if (rc) return rc;
-    h->ec_blocks_data = bd;
-    h->ec_blocks = nb;
-  }
+  if (!h->w || h->ec_blocks == 0) return set_err(h, PWA_ERR_STATE, "no events uploaded");
   std::vector<double> cbuf = consts_block(h, consts);
   long long nd = h->n_data, na = h->n_data + h->n_mc, ld = h->ld;
   unsigned int seq = next_seq(h);
@@ -992,28 +1036,12 @@ int pwa_set_gram_method(pwa_plan* h, int method) {
 }
 
 namespace {
-// Shared memory of one block of pwa_gram_fused and its count of 8 x 8 tiles
-// (GM_* of the device header); 0 bytes where the kernel is compiled empty.
-size_t gram_fused_bytes(const pwa_plan* h, int* tiles) {
-  const int cp = (2 * h->ncol + 7) / 8 * 8, nt = cp / 8;
-  *tiles = nt * (nt + 1) / 2;
-  const size_t bytes = (size_t)h->nout * h->tpb * (cp + 4) * sizeof(double);
-  return bytes <= 104 * 1024 && *tiles <= 12 * (h->tpb / 32) ? bytes : 0;
-}
-
 // The Gram matrix in one pass over the MC events (columns and products in
 // one kernel; block sums in the plan's workspace, summed in block order).
 int gram_fused(pwa_plan* h, const std::vector<double>& cbuf, size_t smem, int tiles,
                cudaStream_t s, std::vector<double>* acc) {
-  CU(cudaFuncSetAttribute((const void*)h->k.gram_fused,
-                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  int per_sm = 0;
-  CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)h->k.gram_fused, h->tpb,
-                                                   smem));
-  if (per_sm < 1) per_sm = 1;
-  const long long want = (long long)per_sm * h->sms, need = (h->n_mc + h->tpb - 1) / h->tpb;
-  int nrows = (int)(want < need ? want : need), ncols = tiles * 64;
-  int rc = ensure_partials(h, (long long)nrows * ncols);
+  int nrows = 0, ncols = tiles * 64;
+  int rc = gram_fused_grid(h, smem, &nrows);
   if (rc) return rc;
   long long beg = h->n_data, end = h->n_data + h->n_mc, ld = h->ld;
   void* a1[] = {(void*)cbuf.data(), &h->xa, &h->xm, &h->w, &beg, &end, &ld, &h->partials};
