@@ -697,9 +697,11 @@ namespace {
 // The n entries of the call numbered h->seq from a mapped result (ll_store:
 // two 8-byte words per entry, the number in each word's upper half) into
 // h->sums.  After limit_s seconds without one of them (a failed launch or a
-// very long kernel), synchronise the stream, which also surfaces launch
-// errors, and look once more; false when the result is not there then.
-bool wait_result(pwa_plan* h, const double* mapped, int n, cudaStream_t s, double limit_s) {
+// very long kernel), synchronise the stream and look once more.  What the
+// synchronisation reports is the error then (`what` names the call), and a
+// result that is not there after it is one too.
+int wait_result(pwa_plan* h, const double* mapped, int n, cudaStream_t s, double limit_s,
+                const char* what) {
   const volatile unsigned long long* m = (const volatile unsigned long long*)mapped;
   const unsigned long long seq = h->seq;
   h->sums.resize(n);
@@ -709,10 +711,14 @@ bool wait_result(pwa_plan* h, const double* mapped, int n, cudaStream_t s, doubl
   for (int j = 0; j < n; ++j) {
     unsigned long long lo = m[2 * j], hi = m[2 * j + 1];
     while (lo >> 32 != seq || hi >> 32 != seq) {
-      if (late) return false;
+      if (late)
+        return set_err(h, PWA_ERR_CUDA, std::string(what) + " did not complete (stale result)");
       if ((++it & 4095u) == 0 &&
           std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count() > limit_s) {
-        cudaStreamSynchronize(s);
+        const cudaError_t e = cudaStreamSynchronize(s);
+        if (e != cudaSuccess)
+          return set_err(h, PWA_ERR_CUDA,
+                         std::string(what) + " did not complete: " + cudaGetErrorString(e));
         late = true;
       }
       lo = m[2 * j];
@@ -721,7 +727,15 @@ bool wait_result(pwa_plan* h, const double* mapped, int n, cudaStream_t s, doubl
     const unsigned long long b = (lo & 0xffffffffull) | (hi << 32);
     std::memcpy(&h->sums[j], &b, sizeof(double));
   }
-  return true;
+  return PWA_OK;
+}
+
+// After a call whose result did not come: the counters back to zero, and its
+// error (with what kept them, if that fails too).
+int reset_counters(pwa_plan* h, int rc, unsigned int* count, long long n) {
+  const cudaError_t e = cudaMemset(count, 0, sizeof(unsigned int) * (size_t)n);
+  if (e != cudaSuccess) h->err += std::string("; counters not reset: ") + cudaGetErrorString(e);
+  return rc;
 }
 
 // A pinned mapped area of `bytes` (host and device address) for the arguments
@@ -755,18 +769,14 @@ int sum_partial_rows(pwa_plan* h, int nrows, int ncols, cudaStream_t s) {
   void* args[] = {&h->partials, &nrows, &ncols, &dp, &seq};
   rc = launch(h, h->k.sum_rows, dim3((unsigned)((ncols + 7) / 8)), dim3(256), args, s);
   if (rc) return rc;
-  if (!wait_result(h, (const double*)hp, ncols, s, 1.0))
-    return set_err(h, PWA_ERR_CUDA, "sums did not arrive (stale result)");
-  return PWA_OK;
+  return wait_result(h, (const double*)hp, ncols, s, 1.0, "sum of block rows");
 }
 
 // The data and MC sums of the last plain, FP32 or floating-shape evaluation.
 int wait_mapped_sums(pwa_plan* h, cudaStream_t s, double* out) {
   const int na2 = 2 * h->nacc;
-  if (!wait_result(h, h->h_map_sc, na2 + 1, s, 1.0)) {
-    cudaMemset(h->ticket, 0, kTicketWords * sizeof(unsigned int));
-    return set_err(h, PWA_ERR_CUDA, "evaluation did not complete (stale result)");
-  }
+  const int rc = wait_result(h, h->h_map_sc, na2 + 1, s, 1.0, "evaluation");
+  if (rc) return reset_counters(h, rc, h->ticket, kTicketWords);
   if (h->sums[na2] != 0.0) return set_err(h, PWA_ERR_CUDA, "evaluation: error flag set");
   std::copy(h->sums.begin(), h->sums.begin() + na2, out);
   return PWA_OK;
@@ -1324,10 +1334,8 @@ int pwa_eval_cached_enqueue(pwa_plan* h, const double* ck, void* stream) {
 // host memory without a stream synchronisation.
 int cached_result(pwa_plan* h, cudaStream_t s, const double** sums, double limit_s = 1.0) {
   const int na = 1 + 2 * h->ncol;
-  if (!wait_result(h, h->h_map, na + 1, s, limit_s)) {
-    cudaMemset(h->ticket, 0, kTicketWords * sizeof(unsigned int));
-    return set_err(h, PWA_ERR_CUDA, "cached evaluation did not complete (stale result)");
-  }
+  const int rc = wait_result(h, h->h_map, na + 1, s, limit_s, "cached evaluation");
+  if (rc) return reset_counters(h, rc, h->ticket, kTicketWords);
   if (h->sums[na] != 0.0)
     return set_err(h, PWA_ERR_CUDA, "cached evaluation: a barrier wait timed out");
   *sums = h->sums.data();
@@ -1871,17 +1879,20 @@ int pwa_pieces_multi(pwa_plan* h, int n_req, const long long* first_tile, const 
     rc = pieces_before(h, &zs[nc * r], &phs[nc * r], ck + 2 * K * (size_t)r, sw[r], mc_share,
                        J.data() + h->jac.size() * r, out + (size_t)r * (3 + 2 * P));
   const auto w0 = std::chrono::steady_clock::now();
+  cudaError_t sync = cudaSuccess;
   for (unsigned it = 1; *mark != (double)seq; ++it)
     if ((it & 4095u) == 0 &&
         std::chrono::duration<double>(std::chrono::steady_clock::now() - w0).count() > 1.0) {
-      CU(cudaStreamSynchronize(s));
+      sync = cudaStreamSynchronize(s);
       break;
     }
   std::atomic_thread_fence(std::memory_order_acquire);
-  if (*mark != (double)seq) {
-    cudaMemset(d_count, 0, sizeof(unsigned int) * h->mcount_cap);
-    return set_err(h, PWA_ERR_CUDA, "batch evaluation did not complete (stale result)");
-  }
+  if (sync != cudaSuccess || *mark != (double)seq)
+    return reset_counters(
+        h, set_err(h, PWA_ERR_CUDA, std::string("batch evaluation did not complete") +
+                                        (sync != cudaSuccess ? std::string(": ") + cudaGetErrorString(sync)
+                                                             : std::string(" (stale result)"))),
+        d_count, h->mcount_cap);
   if (rc) return rc;
   for (int r = 0; r < n_req; ++r)
     pieces_after(h, J.data() + h->jac.size() * r, h_res + (size_t)r * NA,
