@@ -3,6 +3,7 @@ refuses the synchronisation that ends a wait (nothing runs, nothing faults):
 every call that returns sums raises with that reason, and the plan evaluates
 afterwards exactly as before."""
 import ctypes
+import time
 
 import numpy as np
 import pytest
@@ -86,3 +87,22 @@ def test_reason_reported(calls, kind):
         with pytest.raises(PWAError, match="captur"):
             call(stream.cuda_stream)
     np.testing.assert_array_equal(_flat(call(stream.cuda_stream)), before)
+
+
+@pytest.mark.parametrize("kind", ("hessian", "gram", "batch"))
+def test_capture_refused_at_once(calls, kind):
+    """Set-up and service calls synchronise in any case: they refuse a stream
+    under capture without polling for a result first (evaluations poll for up
+    to a second)."""
+    import torch
+
+    from tf_pwa_b200.engine import PWAError
+
+    call, stream = calls[kind], torch.cuda.Stream()
+    call(stream.cuda_stream)
+    with _Capture(stream):
+        t0 = time.perf_counter()
+        with pytest.raises(PWAError):
+            call(stream.cuda_stream)
+        dt = time.perf_counter() - t0
+    assert dt < 0.5, dt

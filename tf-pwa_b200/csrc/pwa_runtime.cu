@@ -758,6 +758,15 @@ int pinned_io(pwa_plan* h, size_t bytes, char** hp, char** dp) {
   return PWA_OK;
 }
 
+// Seconds to poll for a result on stream s before synchronising it: none where
+// s is under capture, as nothing launched there runs and the synchronisation
+// says so at once.
+double poll_limit(cudaStream_t s) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  const cudaError_t e = cudaStreamIsCapturing(s, &st);
+  return e == cudaSuccess && st == cudaStreamCaptureStatusNone ? 1.0 : 0.0;
+}
+
 // Column sums of `nrows` rows of `ncols` in h->partials (pwa_sum_rows), through
 // mapped memory into h->sums: no copy and no stream synchronisation.
 int sum_partial_rows(pwa_plan* h, int nrows, int ncols, cudaStream_t s) {
@@ -769,7 +778,7 @@ int sum_partial_rows(pwa_plan* h, int nrows, int ncols, cudaStream_t s) {
   void* args[] = {&h->partials, &nrows, &ncols, &dp, &seq};
   rc = launch(h, h->k.sum_rows, dim3((unsigned)((ncols + 7) / 8)), dim3(256), args, s);
   if (rc) return rc;
-  return wait_result(h, (const double*)hp, ncols, s, 1.0, "sum of block rows");
+  return wait_result(h, (const double*)hp, ncols, s, poll_limit(s), "sum of block rows");
 }
 
 // The data and MC sums of the last plain, FP32 or floating-shape evaluation.
@@ -1879,10 +1888,11 @@ int pwa_pieces_multi(pwa_plan* h, int n_req, const long long* first_tile, const 
     rc = pieces_before(h, &zs[nc * r], &phs[nc * r], ck + 2 * K * (size_t)r, sw[r], mc_share,
                        J.data() + h->jac.size() * r, out + (size_t)r * (3 + 2 * P));
   const auto w0 = std::chrono::steady_clock::now();
+  const double limit_s = poll_limit(s);
   cudaError_t sync = cudaSuccess;
   for (unsigned it = 1; *mark != (double)seq; ++it)
     if ((it & 4095u) == 0 &&
-        std::chrono::duration<double>(std::chrono::steady_clock::now() - w0).count() > 1.0) {
+        std::chrono::duration<double>(std::chrono::steady_clock::now() - w0).count() > limit_s) {
       sync = cudaStreamSynchronize(s);
       break;
     }
