@@ -28,6 +28,7 @@
 
 #include "../../include/pwa_b200.h"
 #include "pwa_hostprog.h"
+#include "pwa_scratch.h"
 
 namespace {
 
@@ -109,8 +110,7 @@ struct pwa_plan {
   // launches; arguments; rows) and, for batches beyond pin_batch_cap bytes,
   // a pinned block of its own (arguments, then the mapped result)
   char* d_multi = nullptr;
-  long long mcount_cap = 0, mrows_cap = 0;
-  size_t mmeta_cap = 0;
+  BatchScratch mcap;  // its sizes
   char *h_mbig = nullptr, *d_mbig = nullptr;
   size_t mbig_cap = 0;
   int multi_bps = 0;  // blocks per SM of pwa_eval_multi (0: occupancy limit)
@@ -1841,24 +1841,19 @@ int pwa_pieces_multi(pwa_plan* h, int n_req, const long long* first_tile, const 
   const long long n_rows = (n_chunks * NW + n_groups) * NA;
   // grow scratch (serving set-up; steady state allocates nothing)
   const long long n_count = n_groups + n_req + 1;
-  if (n_rows > h->mrows_cap || n_count > h->mcount_cap || words * 8 > h->mmeta_cap) {
+  if (!h->mcap.holds(n_count, words * 8, n_rows)) {
+    const BatchScratch cap = h->mcap.grown(n_count, words * 8, n_rows);
     if (h->d_multi) cudaFree(h->d_multi);
     h->d_multi = nullptr;
-    h->mrows_cap = h->mcount_cap = 0;
-    h->mmeta_cap = 0;
-    const long long cc = (2 * n_count + 63) / 64 * 64, cr = 2 * n_rows;
-    const size_t cm = 2 * meta_bytes;
-    if (cudaMalloc(&h->d_multi, sizeof(unsigned int) * cc + cm + sizeof(double) * cr) !=
-        cudaSuccess)
+    h->mcap = BatchScratch();
+    if (cudaMalloc(&h->d_multi, cap.bytes()) != cudaSuccess)
       return set_err(h, PWA_ERR_OOM, "cudaMalloc of the batch scratch failed");
-    CU(cudaMemsetAsync(h->d_multi, 0, sizeof(unsigned int) * cc, s));
-    h->mcount_cap = cc;
-    h->mmeta_cap = cm;
-    h->mrows_cap = cr;
+    CU(cudaMemsetAsync(h->d_multi, 0, sizeof(unsigned int) * cap.counters, s));
+    h->mcap = cap;
   }
   unsigned int* d_count = (unsigned int*)h->d_multi;
-  char* d_meta = h->d_multi + sizeof(unsigned int) * h->mcount_cap;
-  double* d_rows = (double*)(d_meta + h->mmeta_cap);
+  char* d_meta = h->d_multi + sizeof(unsigned int) * h->mcap.counters;
+  double* d_rows = (double*)(d_meta + h->mcap.args);
   double *h_res = (double*)(h_io + meta_bytes), *d_res = (double*)(d_io + meta_bytes);
   const size_t nc = h->n_coup;
   std::vector<cplx> zs(nc * n_req), phs(nc * n_req);
@@ -1902,7 +1897,7 @@ int pwa_pieces_multi(pwa_plan* h, int n_req, const long long* first_tile, const 
         h, set_err(h, PWA_ERR_CUDA, std::string("batch evaluation did not complete") +
                                         (sync != cudaSuccess ? std::string(": ") + cudaGetErrorString(sync)
                                                              : std::string(" (stale result)"))),
-        d_count, h->mcount_cap);
+        d_count, h->mcap.counters);
   if (rc) return rc;
   for (int r = 0; r < n_req; ++r)
     pieces_after(h, J.data() + h->jac.size() * r, h_res + (size_t)r * NA,
