@@ -1019,8 +1019,10 @@ class ModelCode:
                  "    cpx<double>* __restrict__ e) {\n  using R = double;")
         L += body
         L.append("}\n")
-        # the same with each value times its log-derivatives
-        L.append("template <typename R, bool LDG = true>\n__device__ __forceinline__ void model_shapes(\n"
+        # the same with each value times its log-derivatives: the reference of
+        # the host tests (the kernels apply these constants to their sums)
+        L.append("#ifndef __CUDACC__\n"
+                 "template <typename R, bool LDG = true>\n__device__ __forceinline__ void model_shapes(\n"
                  "    const Consts& C, const double* __restrict__ XM, long long ld, long long i,\n"
                  "    cpx<R>* __restrict__ BW, cpx<R>* __restrict__ DM, cpx<R>* __restrict__ DG) {\n"
                  f"  cpx<R> bw[{max(len(self.shape_res), 1)}], e[{max(len(self.shape_res), 1)}];\n"
@@ -1033,7 +1035,7 @@ class ModelCode:
                 L.append(f"    DG[{si}].re += {ig};")
             L.append(f"    DM[{si}] = cscale(bw[{si}], -2.0 * sqrt({m0}));\n"
                      f"    cfma(DM[{si}], {kap}, be); }}")
-        L.append("}\n")
+        L.append("}\n#endif\n")
         nch, nsr = len(self.group), len(self.shape_res)
         L.append(f"#define PWA_NCHAIN {nch}\n#define PWA_NSRES {nsr}\n"
                  f"#define PWA_SHAPE_CACHE_OK {1 if self.shape_cache_ok else 0}")

@@ -509,15 +509,17 @@ struct DenseColumns {
   }
 };""")
         for wrap, name in (("model_columns", "model_cols"), ("model_columns_ns", "model_cols_ns")):
-            L.append(f"template <typename R, bool LDG = true>\n__device__ __forceinline__ void {wrap}(\n"
-                     "    const Consts& C, const R* __restrict__ XA, const double* __restrict__ XM,\n"
-                     "    long long ld, long long i, cpx<R>* __restrict__ F) {\n"
-                     "  double sp[PWA_NSP];\n"
-                     "  for (int j = 0; j < PWA_NSP; ++j) sp[j] = sqrt(fabs(C.v[pwa_sp_const[j]]));\n"
-                     "  for (int j = 0; j < PWA_NCOL * PWA_NOUT; ++j) F[j] = cmk<R>(R(0), R(0));\n"
-                     "  DenseColumns s{F};\n"
-                     f"  {name}<LDG>(C, sp, XA, XM, ld, i, s);\n"
-                     "}\n")
+            fn = (f"template <typename R, bool LDG = true>\n__device__ __forceinline__ void {wrap}(\n"
+                  "    const Consts& C, const R* __restrict__ XA, const double* __restrict__ XM,\n"
+                  "    long long ld, long long i, cpx<R>* __restrict__ F) {\n"
+                  "  double sp[PWA_NSP];\n"
+                  "  for (int j = 0; j < PWA_NSP; ++j) sp[j] = sqrt(fabs(C.v[pwa_sp_const[j]]));\n"
+                  "  for (int j = 0; j < PWA_NCOL * PWA_NOUT; ++j) F[j] = cmk<R>(R(0), R(0));\n"
+                  "  DenseColumns s{F};\n"
+                  f"  {name}<LDG>(C, sp, XA, XM, ld, i, s);\n"
+                  "}\n")
+            # the kernels take the shape-free columns through sinks of their own
+            L.append(fn if wrap == "model_columns" else f"#ifndef __CUDACC__\n{fn}#endif\n")
         return "\n".join(L)
 
 
