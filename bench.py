@@ -15,6 +15,10 @@ dominant kernel (the fused data-term kernel), timed with CUDA events on the
 stream it is launched on.  ``cpu_baseline`` times the FP64 CPU oracle on a
 bounded sample of the same workload with all host cores.
 
+The printed line holds what identifies and judges the run, a few kilobytes
+that a log's tail keeps whole; ``--details FILE`` writes the full record
+(every form, variant table, Hessian, checks, per-workload rooflines) as JSON.
+
 Multi-GPU (torchrun, one process per GPU): every rank holds its own full
 workload shard (weak scaling); the per-evaluation FP64 sums are combined
 with one NCCL all-reduce before the host forms NLL and gradient.
@@ -805,8 +809,54 @@ def measure_floating(name, args, rank, world, dist, timed, log, n_sig, n_mc, n_b
     return line
 
 
+def _rounded(x):
+    """Floats to 6 significant digits, in dicts and lists too."""
+    if isinstance(x, dict):
+        return {k: _rounded(v) for k, v in x.items()}
+    if isinstance(x, (list, tuple)):
+        return [_rounded(v) for v in x]
+    return float(f"{x:.6g}") if isinstance(x, float) else x
+
+
+def _pick(d, *keys):
+    return {k: d[k] for k in keys if isinstance(d, dict) and k in d}
+
+
+def _printed(line):
+    """The part of a record that is printed: every key of the headline
+    metric (its two numbers in full), the roofline, clocks and baselines
+    without their prose, and one short dict per other workload."""
+    out = _pick(line, "metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step",
+                "higher_is_better", "scaling", "vs_baseline", "dtype", "data", "gpu_launches",
+                "config")
+    roof = ("bound", "achieved", "peak", "unit", "frac", "peak_kind", "traffic", "launch_us")
+    rest = {}
+    for k in ("e2e", "clocks", "cpu_baseline"):
+        if k in line:
+            rest[k] = line[k]
+    if "roofline" in line:
+        rest["roofline"] = _pick(line["roofline"], "kernel", *roof)
+    if "plain_f64" in line:
+        rest["plain_f64"] = _pick(line["plain_f64"], "value", "unit", "ms_per_step")
+    if "check" in line:
+        rest["check"] = _pick(line["check"], "dnll", "grad_max_rel")
+    if "workloads" in line:
+        rest["workloads"] = {
+            name: {**_pick(w, "metric", "value", "unit", "ms_per_step"),
+                   "e2e": w["e2e"]["value"], "plain_f64": w["plain_f64"]["value"],
+                   "roofline": _pick(w["roofline"], "bound", "frac", "launch_us"),
+                   "clocks": w.get("clocks")} if isinstance(w, dict) else w
+            for name, w in line["workloads"].items()}
+    if "serving" in line:
+        sv = line["serving"]
+        rest["serving"] = {"unit": sv["unit"], **{
+            k: {q: v for q, v in sv[k].items() if isinstance(v, (int, float))}
+            for k in ("saturated", "arrivals_over_1s")}}
+    return {**out, **_rounded(rest)}
+
+
 def _compact(line):
-    """A workload's line trimmed for the `workloads` key of the headline line."""
+    """A workload's line trimmed for the `workloads` key of the full record."""
     keep = ("metric", "value", "unit", "ms_per_step", "config", "plain_f64", "fp32_recompute",
             "e2e", "roofline", "host", "autotune", "hessian", "check", "clocks", "setup_s")
     return {k: line[k] for k in keep if k in line}
@@ -869,6 +919,8 @@ def main():
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--headline-only", action="store_true",
                     help="skip the four-body, floating-shape and serving keys")
+    ap.add_argument("--details", metavar="FILE", default=None,
+                    help="write the full record of the run to FILE (JSON)")
     ap.add_argument("--serving", action="store_true",
                     help="run the toy-fit serving workload instead (separate JSON line)")
     ap.add_argument("--n-fits", type=int, default=512)
@@ -939,7 +991,10 @@ def main():
         except Exception as e:  # reported, never fatal
             line["cpu_baseline"] = {"error": repr(e)}
     if rank == 0:
-        print(json.dumps(line), flush=True)
+        if args.details:
+            with open(args.details, "w") as f:
+                json.dump(line, f, indent=1)
+        print(json.dumps(_printed(line)), flush=True)
     if dist is not None:
         dist.barrier()
         dist.destroy_process_group()
