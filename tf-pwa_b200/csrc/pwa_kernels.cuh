@@ -14,9 +14,10 @@
 //               MC:    sum w f,            sum w G_k,             ... d-shape
 //             (the NLL of tf_pwa/model/model.py:407-449 and its gradient
 //             pieces), reduces them with warp shuffles and one shared-memory
-//             stage, and writes one row of block partials.
-// pwa_reduce  sums the block partials in a fixed order (one warp per
-//             accumulator), so results are bitwise reproducible.
+//             stage, and sums the blocks' rows in a fixed order in the same
+//             launch (grouped_publish), so results are bitwise reproducible.
+//             Launched without counters it leaves one row per block to
+// pwa_reduce  which sums them in a fixed order, one warp per accumulator.
 // pwa_pdf_*   per-event sum |A|^2 (the forward amplitude, AbsPDF.__call__).
 // pwa_gram_fused   block partials of M_kl = sum_i w_i sum_o conj(F_ik,o) F_il,o,
 //                  columns and products in one kernel.
@@ -432,7 +433,7 @@ __device__ __forceinline__ void stage_sp(const Consts& C, double* s_sp) {
 // (columns to memory, 480 B per four-body event, then one thread per (k, l)
 // reading two operands per product from shared memory, and a 256 MB buffer
 // allocated and freed per call): a whole fit set-up, column cache of 3e5 and
-// Gram of 1.2e6 four-body events, took 5.1 ms and takes 0.58 ms.  Models
+// Gram of 1.2e6 four-body events, took 5.1 ms and takes 0.57 ms.  Models
 // whose tile exceeds GM_MAX_BYTES (many helicities x columns: two blocks
 // would not fit on an SM) keep that form.
 #define GM_CP ((2 * PWA_NCOL + 7) / 8 * 8)
@@ -942,10 +943,10 @@ extern "C" __global__ void __launch_bounds__(PWA_TPB)
 // no polarised parent and no CP-violating totals (PWA_SHAPE_CACHE_OK), a
 // column factorises as
 //   F_k,o(event) = r_k BW_ch(k)(m; shapes) Fhat_k,o(event):
-// Fhat is the column without its chain's lineshapes (model_columns_ns, in
+// Fhat is the column without its chain's lineshapes (model_cols_ns, in
 // FP64 at the shape setting of the cache, stored FP32 in the tile layout of
 // the cached kernels, for data and MC events), BW the product of the
-// chain's lineshapes from the event's masses (model_shapes, FP64), and r_k
+// chain's lineshapes from the event's masses (model_bw, FP64), and r_k
 // the ratio of the column's barrier normalisations (sqrt(Pz0_l) norm_l per
 // vertex) now and at the cache's setting (host).  An evaluation reads the
 // columns and the masses and produces the sums of pwa_eval_f64 -- S0, the
@@ -977,9 +978,13 @@ struct CRatio {
   double c[2 * PWA_NCOL];  // r_k times the column couplings
 };
 
-// Blocks per SM: the sums of a model set the registers.  Whole evaluations of
-// 2e6 events: D -> K pi pi (9 sums) 57.0 us at 4, 57.7 at 5, 58.8 at 6, 62.9
-// at 8; Lambda_c (23) 155 us at 2, 178 at 3.
+// Blocks per SM: the sums of a model set the registers.  Evaluations of 2e6
+// events with the device idle before each: D -> K pi pi (9 sums) 56 us at
+// two, three and four, 56 to 65 at five, 57 to 62 at six; D -> K pi pi with
+// three resonances (13 sums) 84 to 90 at two and three, 79 at four; Lambda_c
+// (23, 2.1e6 events) 162 at two, 185 at three.  The line at 12 leaves the
+// model of 13 sums at two, where four would be 6 to 12 % faster; no shipped
+// model that takes this kernel has 14 to 22.
 #ifndef PWA_SC_MINB
 #define PWA_SC_MINB (PWA_NACC <= 12 ? 4 : 2)
 #endif
@@ -1045,7 +1050,7 @@ extern "C" __global__ void __launch_bounds__(PWA_TPB, PWA_SC_MINB)
   const int lane_s = threadIdx.x & 31, warp_s = threadIdx.x >> 5;
   const long long stride = (long long)nb * PWA_TPB;
   // segments of 32 events from a multiple of 32 at or below beg (events
-  // outside [beg, end) are computed but not summed)
+  // outside [beg, end) are copied but skipped)
   long long s = staged ? (beg & ~31LL) + (long long)b * PWA_TPB + 32 * warp_s : end;
   if (s < end) sc_issue(sc_smem, Fc, XM, W, ld, s, warp_s, lane_s);
   cp_async_commit();
@@ -1222,11 +1227,15 @@ extern "C" __global__ void __launch_bounds__(PWA_TPB, PWA_SC_MINB)
 // halves for data and MC blocks, result in mapped memory, one launch.
 // Bound: the FP64 pipe and its latency at three blocks per SM (shared
 // memory).  Measured against pwa_eval_f64 and its reduce launch, whole
-// evaluations: four-body 1e6 events 217 vs 1098 us, Lambda_c 2.1e6 379 vs
-// 655 us, D -> K pi pi 1.1e5 20 vs 29 us.
+// evaluations back to back: four-body 1e6 events 218 vs 1098 us, Lambda_c 2.1e6
+// 373 vs 655 us, D -> K pi pi 1.1e5 20 vs 29 us.
 // Models with a density matrix, per-charge totals or more pairs than fit
 // (EC_MAX_BYTES) keep pwa_eval_f64, as do evaluations with free masses or
 // widths, which need the lineshape sums.
+// EC_MINB: as many blocks as the shared memory allows, up to three.  With the
+// device idle before each call: four-body 229 us at three, 252 at two;
+// Lambda_c 383 and 377 to 382; D -> K pi pi, 2e6 events, 68 to 74 at two,
+// three, four and six (no difference beyond the runs').
 #define EC_NW (PWA_TPB / 32)
 #define EC_KW ((PWA_NCOL + EC_NW - 1) / EC_NW)
 #define EC_MAX_BYTES (110 * 1024)
@@ -1387,9 +1396,10 @@ __device__ __forceinline__ void stage_couplings(const CCoup& c, double* s_c) {
 // one event of the current tile from shared memory in FP64; a block
 // barrier frees the stage for the next copy.  Block partials go to
 // `partials`; the last block to finish (atomic ticket) sums them in a fixed
-// order and writes out[0 .. NA), out[NA] = error flag (0 = ok, 1 = a
-// barrier wait gave up) and out[NA+1] = seq (the caller's call number, to
-// detect a stale result); `out` may be mapped host memory.
+// order into the entries 0 .. NA - 1 of `out` (mapped host memory) and the
+// error flag (0 = ok, 1 = a barrier wait gave up) into entry NA; each entry
+// carries the call's number seq (ll_store), so that the host tells it from an
+// earlier call's.
 extern "C" __global__ void __launch_bounds__(PWA_TPB)
     pwa_eval_cached(const CCoup c, const float2* __restrict__ Fc, const double* __restrict__ Wc,
                     long long ntiles, double* __restrict__ partials,
@@ -2632,12 +2642,18 @@ extern "C" __global__ void __launch_bounds__(PWA_TPB, PWA_HESS_MINB)
 // (chunk, warp), then per group.  count: group counters, request counters,
 // finished requests (zero between launches).
 //
-// Bound: at few pairs per event (D -> K pi pi: 24 bytes) by the issue slots
-// and latency of the events' chains (logarithm, division), so eight blocks
-// share an SM (whole rounds of 256 fits, 1.6e7 events: 253 us; 336 at six,
-// 423 at four; loading the next tile ahead costs registers and gains
-// nothing, 282).  With a work list from the host, a row per tile summed in a
-// second launch and the sums copied back, a round took 440 us and takes 226.
+// Bound: latency.  D -> K pi pi (2 pairs, 24 bytes an event), 32 warps on an
+// SM: 56 % of the issue slots used, the warps wait for their loads (4.4 of the
+// 11 cycles between two instructions of a warp) and for the events' chains
+// (logarithm, division: 2.4); FP64 pipe 29 %, DRAM 1.7 TB/s.  Eight blocks
+// share an SM: rounds of 256 fits, 1.6e7 events, with the device idle before
+// each, 241 us at eight, 242 at ten, 262 at six, 287 to 298 at four; with
+// three pairs and two passes (D+ -> K pi pi) 270 to 281, 274, 290, 316.
+// Models of more than eight pairs take the cached kernel's four (none between
+// was measured: the shipped ones have 2, 3 or 9 and more).  Back to back a
+// round takes 228 us; with a work list from the host, a row per tile summed
+// in a second launch and the sums copied back it took 440.  Loading the next
+// tile ahead costs registers and gained nothing.
 #define PWA_MGROUP 8
 #ifndef PWA_MULTI_MINB
 #define PWA_MULTI_MINB (PWA_NF <= 8 ? 8 : PWA_WRED_MINB)
@@ -2805,16 +2821,18 @@ extern "C" __global__ void __launch_bounds__(PWA_TPB, PWA_MULTI_MINB)
 // as they are, without a transposed copy; pairs = 1: components adjacent and
 // 16-byte aligned (two 16-byte loads a final).  Bound: FP64 arithmetic and
 // its latency (two atan2 and two reciprocal square roots per decay).
-// 1e6 four-body events, whole call: 192 us; 1.41 ms with the copy, the axes
-// of every daughter of every topology normalised step by step and all fields
-// held to the end in 255 registers.
+// 1e6 four-body events, calls back to back: 191 us; 1.41 ms with the copy, the
+// axes of every daughter of every topology normalised step by step and all
+// fields held to the end in 255 registers.
 struct FieldRows {  // field j of one event straight to its row
   double* p;
   long long ld;
   __device__ __forceinline__ double& operator[](int j) const { return p[j * ld]; }
 };
-// three blocks per SM: four-body 203 us against 248 at two and 204 at four
-// (D -> K pi pi 103, 129 and 92)
+// Blocks per SM, 1e6 events, the device idle before each call (four-body /
+// Lambda_c / D -> K pi pi): two 246 / 391 / 130 us, three 202 / 341 / 103,
+// four 204 / 325 / 92, five 213 / 328 / 93.  Three is the four-body model's
+// best; the three-body models would gain 5 and 10 % at four.
 #ifndef PWA_KIN_MINB
 #define PWA_KIN_MINB 3
 #endif

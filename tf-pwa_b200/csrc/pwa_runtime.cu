@@ -87,13 +87,14 @@ struct pwa_plan {
   int cached_variant = -1;
   size_t cached_smem = 0;
   unsigned int* ticket = nullptr;  // [0] finished groups, [1] error flag, [2 + g] group counts
-  // one pinned mapped block: the results below, and pin_batch_cap bytes from
-  // pin_batch for pwa_pieces_multi
+  // one pinned mapped block: the results below (two words an entry, ll_store),
+  // and pin_batch_cap bytes from pin_batch for the arguments and results of
+  // batches, Hessian and Gram sums
   char *h_pin = nullptr, *d_pin = nullptr;
   size_t pin_batch = 0, pin_batch_cap = 0;
-  double* h_map = nullptr;         // mapped pinned result of the cached kernel
-  double* d_map = nullptr;         // its device address
-  double* h_map_sc = nullptr;      // mapped result of pwa_eval_shapecache (2 nacc + 2)
+  double* h_map = nullptr;     // result of the cached kernels: 1 + 2 ncol sums, error flag
+  double* d_map = nullptr;     // its device address
+  double* h_map_sc = nullptr;  // of plain, FP32 and floating-shape evaluations: 2 nacc, flag
   double* d_map_sc = nullptr;
   unsigned int seq = 0;          // number of the last call with a mapped result, never 0 after one
   std::vector<double> sums;      // the last such result and its error flag
