@@ -1222,14 +1222,16 @@ int pwa_cache_data(pwa_plan* h, const double* consts, void* stream) {
   if (rc) return rc;
   // streaming kernel: PWA_STAGES tiles of (nf float2 + 1 double) per event in
   // shared memory per block.  The ring variants (0, 3) exist only where their
-  // tiles fit in a block's shared memory (0 blocks otherwise; launches of
-  // them then run variant 2)
+  // tiles fit in a block's shared memory beside the kernel's own arrays (0
+  // blocks otherwise; launches of them then run variant 2)
   int smem_optin = 0;
   CU(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device));
   const int stages = 3;
   h->cached_smem = (size_t)stages * tile * (h->nf * sizeof(float2) + sizeof(double));
   h->cached_blocks = 0;
-  if (h->cached_smem + 2048 <= (size_t)smem_optin) {
+  cudaFuncAttributes ring;
+  CU(cudaFuncGetAttributes(&ring, (const void*)h->k.eval_cached));
+  if (h->cached_smem + ring.sharedSizeBytes <= (size_t)smem_optin) {
     CU(cudaFuncSetAttribute((const void*)h->k.eval_cached,
                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h->cached_smem));
     int per_sm = 0;
@@ -1255,7 +1257,8 @@ int pwa_cache_data(pwa_plan* h, const double* consts, void* stream) {
   // ring with register-light consumers: 2 stages (PWA_RSTAGES) per block
   h->cached_smem_ring2 = (size_t)2 * tile * (h->nf * sizeof(float2) + sizeof(double));
   h->cached_blocks_ring2 = 0;
-  if (h->cached_smem_ring2 + 2048 <= (size_t)smem_optin) {
+  CU(cudaFuncGetAttributes(&ring, (const void*)h->k.eval_cached_ring2));
+  if (h->cached_smem_ring2 + ring.sharedSizeBytes <= (size_t)smem_optin) {
     CU(cudaFuncSetAttribute((const void*)h->k.eval_cached_ring2,
                             cudaFuncAttributeMaxDynamicSharedMemorySize,
                             (int)h->cached_smem_ring2));
