@@ -1464,8 +1464,9 @@ class Engine:
                                                          int(bps)), "pwa_set_cached_config")
 
     def set_gram_method(self, method):
-        """0: FP64 Gram on the CUDA cores; 1: tensor cores (int8 slices,
-        exact integer accumulation); -1: automatic."""
+        """0: FP64 matrix instructions in the kernel that forms the columns
+        (CUDA cores where its tile exceeds a block's shared memory); 1: tensor
+        cores (int8 slices, exact integer accumulation); -1: automatic (0)."""
         self._check(load_library().pwa_set_gram_method(self.h, int(method)),
                     "pwa_set_gram_method")
 
